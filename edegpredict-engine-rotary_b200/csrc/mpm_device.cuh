@@ -93,6 +93,7 @@ template <typename R> struct alignas(128) Inst {
     R D1, D2, D3, D4c, D5, Dth;
     R Tspan;                       // max(Tm - Tamb, 1)
     R ylo;                         // lower bound of the flow stress of an unheated particle (0: none)
+    R ymin;                        // ylo min(m, 1): times 1 - Ts, a lower bound at any temperature (0: none)
     R dTmax;                       // Tm - Tamb (temperature cap as a rise)
     R heat;                        // beta / max(rho_phys cp, 1e-12)
     R apic;                        // apic_dinv_factor, applied as factor/dx
@@ -183,9 +184,10 @@ template <typename R> struct alignas(128) Inst {
     double esc_scale;
 };
 
-// Deterministic mode: node-tile values stored per work item (channels m,
-// p_x, p_y, p_z, T m; kTileNodes nodes each, in tile order x + 6y + 36z).
+// Deterministic mode: node-tile values stored per work item (kTileNodes
+// records (m, p_x, p_y, p_z) in tile order x + 6y + 36z, then kTileNodes T m).
 constexpr int kPartCh = 5;
+constexpr int kPartReals = kPartCh * kTileNodes;
 
 // Threads per CTA of the step kernel (four warps, each with its own P2G tile).
 constexpr int kNT = 128;
@@ -209,7 +211,6 @@ struct StepArgs {
     int p2g_step;       // step index of the P2G part
     int ext;            // some instance runs the adiabatic shear model or heat conduction: launches
                         // take the kernel variant that has them (the others carry none of their code)
-    int chunk = 2;         // FP32 particles per pass / 128 (1, 2 or 4): the launch config's pass size
     void* part = nullptr;  // deterministic mode: each work item's node tile is stored at
                            // part + wi * kPartCh * kTileNodes (R values) for k_node_sum to add
                            // up in a fixed order, instead of added to the grid with atomics
@@ -220,9 +221,7 @@ struct StepArgs {
 // Quadratic B-spline weights on one axis, restating getWeightsAndGradients
 // (reference src/MPMSolver.cu:20-34) in cell units: base = floor(xi - 0.5),
 // d = xi - base in [0.5, 1.5); dw is d/dxi (divide by dx for a gradient).
-template <typename R> __device__ __forceinline__ int bspline(R xi, R w[3], R dw[3]) {
-    R fb = floor(xi - R(0.5));
-    R d = xi - fb;
+template <typename R> __device__ __forceinline__ void bspline_at(R d, R w[3], R dw[3]) {
     R a = R(1.5) - d, b = d - R(1), c = d - R(0.5);
     w[0] = R(0.5) * a * a;
     w[1] = R(0.75) - b * b;
@@ -230,6 +229,10 @@ template <typename R> __device__ __forceinline__ int bspline(R xi, R w[3], R dw[
     dw[0] = -a;
     dw[1] = R(-2) * b;
     dw[2] = c;
+}
+template <typename R> __device__ __forceinline__ int bspline(R xi, R w[3], R dw[3]) {
+    const R fb = floor(xi - R(0.5));
+    bspline_at(xi - fb, w, dw);
     return (int)fb;
 }
 

@@ -123,6 +123,7 @@ class Engine final : public EngineBase {
     int* d_ierr = nullptr;         // one error word per instance (ERR_NUMERIC, ERR_NEWTON)
     int64_t ierr_alloc = 0;
     unsigned long long* d_ctr = nullptr;
+    unsigned int* d_ticket = nullptr;   // work-item tickets of the step kernel, zero between launches
     static constexpr size_t kCtrBytes = 4 * sizeof(unsigned long long) + 2 * sizeof(double);
     double *d_stat_part = nullptr, *d_stat_out = nullptr;
     int stat_blocks = 0;
@@ -140,7 +141,7 @@ class Engine final : public EngineBase {
     int64_t launch_base = 0;
     int sort_every = 16, threads = 128, ctas_per_sm = 4, prec_ = MPM_PREC_F32;
     static constexpr int kDefaultPassChunk = 1;
-    int pass_chunk = kDefaultPassChunk;   // FP32 particles per pass of the step kernel / 128
+    int pass_chunk = kDefaultPassChunk;   // the launch config's pass_size / 128 (kept, no effect)
     bool use_graph = false;
     int rbuf = 0;
     // deterministic mode (mpm_launch_config.deterministic): every work item's
@@ -200,7 +201,7 @@ class Engine final : public EngineBase {
                         d_bin_local,
                         d_inst_pbase, d_key, d_rank, d_newbin, d_count, d_offset, d_flag, d_flag_scan, d_scan_tmp,
                         d_pos, d_work, d_nwork, d_err, d_ierr, d_ctr, d_stat_part, d_stat_out, d_stage, d_gen,
-                        d_map, d_perm, d_part, d_esc, d_esc_flag, d_pext, d_flags};
+                        d_map, d_perm, d_part, d_esc, d_esc_flag, d_pext, d_flags, d_ticket};
         for (void* p : ptrs)
             if (p) cudaFree(p);
         for (auto& x : I)
@@ -240,6 +241,8 @@ class Engine final : public EngineBase {
         // then two FP64 sums (contact friction work, contact normal force)
         CK(cudaMalloc(&d_ctr, kCtrBytes));
         CK(cudaMemsetAsync(d_ctr, 0, kCtrBytes, st));
+        CK(cudaMalloc(&d_ticket, 2 * sizeof(unsigned int)));
+        CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned int), st));
         stat_blocks = 148 * 8;   // 8 CTAs per SM of the metrics reduction (more loads in flight)
         CK(cudaMalloc(&d_stat_part, sizeof(double) * kStatSlots * stat_blocks));
         CK(cudaMalloc(&d_stat_out, sizeof(double) * kStatSlots));
@@ -697,6 +700,8 @@ class Engine final : public EngineBase {
             d.ylo = (p.jc_A > 0.0 && p.jc_B >= 0.0 && p.jc_C >= 0.0 && rt_lo > 0.0)
                         ? (R)(p.jc_A * rt_lo * (1.0 - 1e-4))
                         : R(0);
+            // (the same margin again for the rounding of 1 - Ts^m and of the bound)
+            d.ymin = p.jc_m > 0.0 ? (R)((double)d.ylo * std::min(p.jc_m, 1.0) * (1.0 - 1e-4)) : R(0);
         }
         d.dTmax = (R)(p.Tm - p.Tamb);
         d.heat = (R)(p.beta / std::max(p.rho_phys * p.cp, 1e-12));
@@ -1343,7 +1348,6 @@ class Engine final : public EngineBase {
         };
         auto p2g_args = [&](StepArgs a) {
             a.part = det ? d_part : nullptr;
-            a.chunk = pass_chunk;
             return a;
         };
         // heat conduction: the diffusion step on grid buffer b before the G2P that reads it
@@ -1354,7 +1358,7 @@ class Engine final : public EngineBase {
             if ((s = clear(w)) != MPM_OK) return s;
             const StepArgs a = p2g_args(StepArgs{0, 0, N == 1 ? 1 : 0, ext ? 1 : 0, 0, xk});
             launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], a, w, false, true, threads, cps, d_err, d_ctr,
-                           st);
+                           d_ticket, st);
             node_sum(w);
             for (int k = 0; k + 1 < N; ++k) {
                 if ((s = maybe_sort(k)) != MPM_OK) return s;
@@ -1364,7 +1368,7 @@ class Engine final : public EngineBase {
                 const StepArgs b = p2g_args(StepArgs{k, 0, (k + 2 == N) ? 1 : 0, 0, k + 1, xk});
                 prof_begin();
                 launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], b, w, true, true, threads, cps, d_err,
-                               d_ctr, st);
+                               d_ctr, d_ticket, st);
                 prof_end();
                 node_sum(w ^ 1);
                 w ^= 1;
@@ -1375,9 +1379,8 @@ class Engine final : public EngineBase {
             raster_all(N - 1);
             diffuse(w);
             StepArgs c{N - 1, 1, 0, 0, N - 1, xk};
-            c.chunk = pass_chunk;
             launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], c, w, true, false, threads, cps, d_err, d_ctr,
-                           st);
+                           d_ticket, st);
         } else {
             for (int k = 0; k < N; ++k) {
                 if ((s = maybe_sort(k)) != MPM_OK) return s;
@@ -1385,16 +1388,15 @@ class Engine final : public EngineBase {
                 const StepArgs a = p2g_args(StepArgs{k, 0, 1, (ext && k == 0) ? 1 : 0, k, xk});
                 prof_begin();
                 launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], a, w, false, true, threads, cps, d_err,
-                               d_ctr, st);
+                               d_ctr, d_ticket, st);
                 prof_end();
                 node_sum(w);
                 raster_all(k);
                 diffuse(w);
                 StepArgs c{k, 1, 0, 0, k, xk};
-                c.chunk = pass_chunk;
-                prof_begin();
+                    prof_begin();
                 launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], c, w, true, false, threads, cps, d_err,
-                               d_ctr, st);
+                               d_ctr, d_ticket, st);
                 prof_end();
             }
         }

@@ -70,7 +70,8 @@ void launch_heat_diffuse(const Inst<R>* insts, int n_inst, int b, int64_t total,
 template <typename R>
 void launch_step(const Inst<R>* insts, const Work* work, const int* n_work, int max_work, const PState<R>& ps,
                  const StepArgs& a, int rbuf, bool g2p, bool p2g, int threads, int ctas_per_sm, int* err,
-                 unsigned long long* counters, cudaStream_t st);
+                 unsigned long long* counters, unsigned int* ticket, cudaStream_t st);
+// (ticket: two zeroed words of the handle; every launch leaves them zero)
 
 // Deterministic mode: the grid buffer b of every instance from the node
 // tiles the step launch stored per work item (part, part_items items) and the
