@@ -709,55 +709,29 @@ __global__ void k_export(const Inst<R>* inst, PState<R> ps, int64_t pbase, int64
 }
 
 // The particle records (MPMParticle, 504 bytes) in upload order.  A warp takes
-// 32 consecutive slots: each lane loads its particle's fields (coalesced
-// 128-bit loads) into a row of shared memory, then the warp writes the 32
-// records one after the other, lane l the 8-byte words l and l + 32 of each,
-// so that a record leaves as two contiguous stores.  (One thread per record
-// wrote 63 words at a stride of 504 bytes, every store of the warp to 32
-// separate sectors.)  A word is const, field + const or a staged 64-bit
-// value, fixed per lane for the whole kernel.  Bound by memory: 33.5 M FP32
-// records (24.4 GB read and written) take 7.7 ms, 21.0 ms before.
-constexpr int kAosField = 47;   // staged fields of a particle (odd: conflict-free columns)
-constexpr int kAosWide = 5;     // staged 64-bit words: x, y, z, (id, status), (0, asb)
-constexpr int kAosWords = (int)(sizeof(AosParticle) / 8);
-template <typename R> constexpr int kAosThreads = sizeof(R) == 4 ? 128 : 64;   // 30 and 27 KB of shared memory
-
-// Word w of a record: the staged field f (>= 0) or wide word -1 - f that it
-// takes (kAosNone: neither) and the constant added to it.  -0.0 adds nothing,
-// whatever the sign of the field.
-constexpr int kAosNone = 1000;
-struct AosWord {
-    int f;
-    double add;
-};
-__device__ __forceinline__ AosWord aos_word(int w, double rho, double vol, double mass, double Tamb) {
-    if (w < 3) return {-1 - w, 0.0};                                  // x, y, z
-    if (w < 6) return {w - 3, -0.0};                                  // v
-    if (w == 12) return {kAosNone, rho};
-    if (w == 14) return {kAosNone, vol};
-    if (w == 15) return {kAosNone, mass};
-    if (w == 16) return {3, Tamb};
-    if (w >= 17 && w < 26) return {w - 13, (w - 17) % 4 == 0 ? 1.0 : 0.0};   // F = H + I
-    if (w >= 26 && w < 35) return {w - 13, (w - 26) % 4 == 0 ? 1.0 : 0.0};   // F_p
-    if (w >= 35 && w < 60) return {w - 13, -0.0};   // C, stress, backstress, eps, strain rate, damage, residual
-    if (w == 60) return {-4, 0.0};
-    if (w == 62) return {-5, 0.0};
-    return {kAosNone, 0.0};
-}
+// 32 consecutive slots: each lane builds its particle's record as 63 doubles
+// in shared memory from coalesced 128-bit loads, then the warp writes the 32
+// records one after the other, lane l the words l and l + 32 of each, so that
+// a record leaves as two contiguous stores.  (One thread per record writing
+// its 63 words put every store of a warp into 32 separate sectors: 21.0 ms
+// for 33.5 M FP32 records, 24.4 GB read and written.  Staging the FP32 fields
+// and converting in the write loop took 7.7 ms, bound by that loop's chain of
+// shared-memory loads and branches; whole words leave it a load and a store.)
+constexpr int kAosWords = (int)(sizeof(AosParticle) / 8);   // odd: conflict-free columns
+constexpr int kAosThreads = 64;                              // 32 KB of shared memory
 
 template <typename R>
-__global__ void __launch_bounds__(kAosThreads<R>) k_export_aos(const Inst<R>* inst, PState<R> ps, int64_t pbase, int64_t n,
+__global__ void __launch_bounds__(kAosThreads) k_export_aos(const Inst<R>* inst, PState<R> ps, int64_t pbase, int64_t n,
                                                             double Tamb, double rho, AosParticle* out) {
-    __shared__ R sf[kAosThreads<R> / 32][32 * kAosField];
-    __shared__ unsigned long long sw[kAosThreads<R> / 32][32 * kAosWide];
+    __shared__ double rec[kAosThreads / 32][32 * kAosWords];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int64_t s0 = ((int64_t)blockIdx.x * (kAosThreads<R> / 32) + wid) * 32;
+    const int64_t s0 = ((int64_t)blockIdx.x * (kAosThreads / 32) + wid) * 32;
     if (s0 >= n) return;
     const Inst<R>& P = *inst;
     int32_t orig = 0;
     if (s0 + lane < n) {
         const int64_t pi = pbase + s0 + lane;
-        R* f = &sf[wid][lane * kAosField];
+        double* q = &rec[wid][lane * kAosWords];
         const V4<R> a0 = ps.A[0][pi], a1 = ps.A[1][pi], a2 = ps.A[2][pi], a3 = ps.A[3][pi], a4 = ps.A[4][pi],
                     a5 = ps.A[5][pi];
         const V4<R> b0 = ps.B[0][pi], b1 = ps.B[1][pi], b2 = ps.B[2][pi], b3 = ps.B[3][pi];
@@ -765,38 +739,42 @@ __global__ void __launch_bounds__(kAosThreads<R>) k_export_aos(const Inst<R>* in
         V4<R> k0 = mk4<R>(0, 0, 0, 0), k1 = k0;
         if (ps.K[0]) { k0 = ps.K[0][pi]; k1 = ps.K[1][pi]; }
         orig = ps.orig[pi];
+        const unsigned int id = (unsigned int)ps.id[pi], status = ps.status[pi], asb = ps.asb[pi];
+        const R sres = ps.sres[pi];
         double xw[3];
         world_pos(P, ps, pi, a0, xw);
-        f[0] = b0.x; f[1] = b0.y; f[2] = b0.z; f[3] = a3.z;
-        f[4] = a1.x; f[5] = a1.y; f[6] = a1.z; f[7] = a1.w; f[8] = a2.x; f[9] = a2.y; f[10] = a2.z; f[11] = a2.w;
-        f[12] = a3.x;
-        f[13] = a4.x; f[14] = a4.y; f[15] = a4.z; f[16] = a4.w; f[17] = a5.x; f[18] = a5.y; f[19] = a5.z; f[20] = a5.w;
-        f[21] = a3.y;
-        f[22] = b1.x; f[23] = b1.y; f[24] = b1.z; f[25] = b1.w; f[26] = b2.x; f[27] = b2.y; f[28] = b2.z; f[29] = b2.w;
-        f[30] = b3.x;
-        f[31] = s0v.x; f[32] = s0v.y; f[33] = s0v.z; f[34] = s0v.w; f[35] = s1v.x; f[36] = s1v.y;
-        f[37] = k0.x; f[38] = k0.y; f[39] = k0.z; f[40] = k0.w; f[41] = k1.x; f[42] = k1.y;
-        f[43] = a0.w; f[44] = b0.w; f[45] = a3.w; f[46] = ps.sres[pi];
-        unsigned long long* wd = &sw[wid][lane * kAosWide];
-        for (int a = 0; a < 3; ++a) wd[a] = (unsigned long long)__double_as_longlong(xw[a]);
-        wd[3] = (unsigned long long)(uint32_t)ps.id[pi] | ((unsigned long long)ps.status[pi] << 32);
-        wd[4] = (unsigned long long)ps.asb[pi] << 32;
+        q[0] = xw[0]; q[1] = xw[1]; q[2] = xw[2];
+        q[3] = b0.x; q[4] = b0.y; q[5] = b0.z;
+#pragma unroll
+        for (int k = 6; k < 12; ++k) q[k] = 0.0;                      // f, ext_f
+        q[12] = rho; q[13] = 0.0; q[14] = (double)P.pvol; q[15] = (double)P.pmass;
+        q[16] = Tamb + (double)a3.z;
+        const R H[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
+        const R Hp[9] = {a4.x, a4.y, a4.z, a4.w, a5.x, a5.y, a5.z, a5.w, a3.y};
+        const R C[9] = {b1.x, b1.y, b1.z, b1.w, b2.x, b2.y, b2.z, b2.w, b3.x};
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const double id_ = (k % 4 == 0) ? 1.0 : 0.0;
+            q[17 + k] = (double)H[k] + id_;
+            q[26 + k] = (double)Hp[k] + id_;
+            q[35 + k] = (double)C[k];
+        }
+        q[44] = s0v.x; q[45] = s0v.y; q[46] = s0v.z; q[47] = s0v.w; q[48] = s1v.x; q[49] = s1v.y;
+        q[50] = k0.x; q[51] = k0.y; q[52] = k0.z; q[53] = k0.w; q[54] = k1.x; q[55] = k1.y;
+        q[56] = a0.w; q[57] = b0.w; q[58] = a3.w; q[59] = sres;
+        q[60] = __hiloint2double((int)status, (int)id);
+        q[61] = 0.0;                                                  // cellHash, lodZone
+        q[62] = __hiloint2double((int)asb, 0);                        // lastUpdateStep, asbCounter
     }
     __syncwarp();
-    const AosWord w0 = aos_word(lane, rho, (double)P.pvol, (double)P.pmass, Tamb);
-    const AosWord w1 = aos_word(lane + 32, rho, (double)P.pvol, (double)P.pmass, Tamb);
     const int m = (int)(n - s0 < 32 ? n - s0 : 32);
-    auto word = [&](const AosWord& w, int r) -> unsigned long long {
-        if (w.f < 0) return sw[wid][r * kAosWide - 1 - w.f];
-        const double v = w.f == kAosNone ? w.add : (double)sf[wid][r * kAosField + w.f] + w.add;
-        return (unsigned long long)__double_as_longlong(v);
-    };
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < m; ++r) {
         const int32_t o = __shfl_sync(0xffffffffu, orig, r);
-        unsigned long long* dst = reinterpret_cast<unsigned long long*>(out + o);
-        dst[lane] = word(w0, r);
-        if (lane + 32 < kAosWords) dst[lane + 32] = word(w1, r);
+        const double* src = &rec[wid][r * kAosWords];
+        double* dst = reinterpret_cast<double*>(out + o);
+        dst[lane] = src[lane];
+        if (lane + 32 < kAosWords) dst[lane + 32] = src[lane + 32];
     }
 }
 
@@ -1060,8 +1038,8 @@ template <typename R>
 void launch_export_aos(const Inst<R>* inst_dev, const PState<R>& ps, int64_t pbase, int64_t n, double Tamb,
                        double rho, void* out, cudaStream_t st) {
     if (n <= 0) return;
-    constexpr int t = kAosThreads<R>;
-    k_export_aos<R><<<(int)((n + t - 1) / t), t, 0, st>>>(inst_dev, ps, pbase, n, Tamb, rho, (AosParticle*)out);
+    k_export_aos<R><<<(int)((n + kAosThreads - 1) / kAosThreads), kAosThreads, 0, st>>>(inst_dev, ps, pbase, n, Tamb,
+                                                                                        rho, (AosParticle*)out);
     ++launch_counter();
 }
 

@@ -1325,6 +1325,7 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                 // own.  The error word is never cleared: every later status or
                 // metrics call on the handle returns MPM_TIMEOUT, and the
                 // caller is expected to stop using it.
+                if (kStage) async_wait<0>();
                 if (tid == 0) atomicOr(err, ERR_TIMEOUT);
                 return;
             }
