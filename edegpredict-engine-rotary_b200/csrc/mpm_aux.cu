@@ -928,7 +928,15 @@ __global__ void k_stats(const Inst<R>* inst, PState<R> ps, int64_t pbase, int64_
 // One CTA per slot: thread t combines the block partials t, t + kFinalT, ...
 // in order, then a fixed tree over the threads (the same order on every run).
 constexpr int kFinalT = 256;
-__global__ void __launch_bounds__(kFinalT) k_stats_final(const double* partial, int nb, double* out) {
+// Writes the sums, and from CTA 0 the handle's counters and the error words,
+// into pinned host memory: one synchronisation and no copy gives the host all
+// of them (the metrics call of a small workpiece took 85 us with five copies
+// and two synchronisations).
+__global__ void __launch_bounds__(kFinalT) k_stats_final(const double* partial, int nb, ReadBack* out,
+                                                         const unsigned long long* ctr, const int* err,
+                                                         const int* ierr) {
+    if (blockIdx.x == 0 && threadIdx.x < kCounters) out->ctr[threadIdx.x] = ctr[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == kCounters) { out->err = *err; out->ierr = *ierr; }
     __shared__ double sh[kFinalT];
     const int q = blockIdx.x, t = threadIdx.x;
     const bool isMin = (q >= 19 && q < 22);
@@ -947,7 +955,7 @@ __global__ void __launch_bounds__(kFinalT) k_stats_final(const double* partial, 
         }
         __syncthreads();
     }
-    if (t == 0) out[q] = sh[0];
+    if (t == 0) out->stat[q] = sh[0];
 }
 
 template <typename R>
@@ -1055,10 +1063,20 @@ void launch_import_aos(const Inst<R>* inst_dev, const PState<R>& ps, int64_t pba
 
 template <typename R>
 void launch_stats(const Inst<R>* inst_dev, const PState<R>& ps, int64_t pbase, int64_t n, double mu, double K,
-                  double rho, double cp, double Tamb, double* partial, int nblocks, double* out, cudaStream_t st) {
+                  double rho, double cp, double Tamb, double* partial, int nblocks, ReadBack* out,
+                  const unsigned long long* ctr, const int* err, const int* ierr, cudaStream_t st) {
     k_stats<R><<<nblocks, kT, 0, st>>>(inst_dev, ps, pbase, n, mu, K, rho, cp, Tamb, partial);
-    k_stats_final<<<kStatSlots, kFinalT, 0, st>>>(partial, nblocks, out);
+    k_stats_final<<<kStatSlots, kFinalT, 0, st>>>(partial, nblocks, out, ctr, err, ierr);
     launch_counter() += 2;
+}
+
+__global__ void k_read_words(ReadBack* out, const int* err, const int* ierr) {
+    out->err = *err;
+    out->ierr = *ierr;
+}
+void launch_read_words(ReadBack* out, const int* err, const int* ierr, cudaStream_t st) {
+    k_read_words<<<1, 1, 0, st>>>(out, err, ierr);
+    ++launch_counter();
 }
 
 template <typename R>
@@ -1186,7 +1204,8 @@ void launch_heat_diffuse(const Inst<R>* insts, int n_inst, int b, int64_t total,
     template void launch_import_aos<R>(const Inst<R>*, const PState<R>&, int64_t, int64_t, double, uint32_t,         \
                                        const void*, V4<R>*, int*, cudaStream_t);                                     \
     template void launch_stats<R>(const Inst<R>*, const PState<R>&, int64_t, int64_t, double, double, double, double, \
-                                  double, double*, int, double*, cudaStream_t);                                      \
+                                  double, double*, int, ReadBack*, const unsigned long long*, const int*,           \
+                                  const int*, cudaStream_t);                                                         \
     template void launch_set_temps<R>(const PState<R>&, int64_t, int64_t, const double*, int64_t, double, cudaStream_t); \
     template void launch_relayout<R>(const PState<R>&, const PState<R>&, const RelayoutMap*, int, int64_t, cudaStream_t); \
     template void launch_heat_diffuse<R>(const Inst<R>*, int, int, int64_t, cudaStream_t);                      \

@@ -124,8 +124,9 @@ class Engine final : public EngineBase {
     int64_t ierr_alloc = 0;
     unsigned long long* d_ctr = nullptr;
     unsigned int* d_ticket = nullptr;   // work-item tickets of the step kernel, zero between launches
-    static constexpr size_t kCtrBytes = 4 * sizeof(unsigned long long) + 2 * sizeof(double);
-    double *d_stat_part = nullptr, *d_stat_out = nullptr;
+    static constexpr size_t kCtrBytes = kCounters * sizeof(unsigned long long);
+    double* d_stat_part = nullptr;
+    ReadBack* h_rb = nullptr;      // pinned
     int stat_blocks = 0;
     void* d_stage = nullptr;
     size_t stage_bytes = 0;
@@ -200,10 +201,11 @@ class Engine final : public EngineBase {
                         d_key_base, d_bin_key, d_bin_inst,
                         d_bin_local,
                         d_inst_pbase, d_key, d_rank, d_newbin, d_count, d_offset, d_flag, d_flag_scan, d_scan_tmp,
-                        d_pos, d_work, d_nwork, d_err, d_ierr, d_ctr, d_stat_part, d_stat_out, d_stage, d_gen,
+                        d_pos, d_work, d_nwork, d_err, d_ierr, d_ctr, d_stat_part, d_stage, d_gen,
                         d_map, d_perm, d_part, d_esc, d_esc_flag, d_pext, d_flags, d_ticket};
         for (void* p : ptrs)
             if (p) cudaFree(p);
+        if (h_rb) cudaFreeHost(h_rb);
         for (auto& x : I)
             if (x.d_samples) cudaFree(x.d_samples);
         for (auto e : ev_pool) cudaEventDestroy(e);
@@ -245,7 +247,7 @@ class Engine final : public EngineBase {
         CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned int), st));
         stat_blocks = 148 * 8;   // 8 CTAs per SM of the metrics reduction (more loads in flight)
         CK(cudaMalloc(&d_stat_part, sizeof(double) * kStatSlots * stat_blocks));
-        CK(cudaMalloc(&d_stat_out, sizeof(double) * kStatSlots));
+        CK(cudaHostAlloc(&h_rb, sizeof(ReadBack), cudaHostAllocDefault));
         return relayout(std::move(nI), std::vector<int>(n, -1));
     }
 
@@ -862,7 +864,7 @@ class Engine final : public EngineBase {
             mpm_status s = set_tool(i, tool);
             if (s != MPM_OK) return s;
         }
-        const size_t need = 4 * (size_t)(2 * ncand + 2);
+        const size_t need = 4 * (size_t)(2 * ncand + 2 + scan_tmp_size(ncand));
         if (gen_bytes < need) {
             if (d_gen) cudaFree(d_gen);
             d_gen = nullptr;
@@ -871,8 +873,7 @@ class Engine final : public EngineBase {
         }
         int32_t* flag = d_gen;
         int32_t* idx = d_gen + ncand + 1;
-        int32_t* tmp = nullptr;
-        CK(cudaMalloc(&tmp, 4 * scan_tmp_size(ncand)));
+        int32_t* tmp = idx + ncand + 1;
         Inst<R> P = h_inst[i];
         const int tool_check = (tool && tool->mode != MPM_TOOL_NONE) ? 1 : 0;
         launch_gen<R>(P, c0, c1, ppc, seed, instance, fixed_layers, T0 - x.p.Tamb, tool_check, flag, idx, tmp, ps[cur],
@@ -881,7 +882,6 @@ class Engine final : public EngineBase {
         CK(cudaMemcpyAsync(&lastf, flag + ncand - 1, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(&lasti, idx + ncand - 1, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        cudaFree(tmp);
         x.np = (int64_t)lasti + lastf;
         x.fresh = 1;
         x.broken = false;
@@ -1001,8 +1001,7 @@ class Engine final : public EngineBase {
             if (f.dst) CK(cudaMemcpyAsync(f.dst, *f.dev, (size_t)e * n * f.per, cudaMemcpyDeviceToHost, st));
         if (h->status) CK(cudaMemcpyAsync(h->status, o.status, 4 * n, cudaMemcpyDeviceToHost, st));
         if (h->id) CK(cudaMemcpyAsync(h->id, o.id, 4 * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        return inst_status(i);
+        return sync_status(i);
     }
 
     mpm_status export_aos(int i, void* dst, int64_t bytes) override {
@@ -1031,8 +1030,7 @@ class Engine final : public EngineBase {
         }
         launch_export_aos<R>(d_inst + i, ps[cur], x.pbase, x.np, x.p.Tamb, x.p.rho_phys, out, st);
         if (!dev) CK(cudaMemcpyAsync(dst, out, (size_t)504 * x.np, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        return inst_status(i);
+        return sync_status(i);
     }
 
     mpm_status import_aos(int i, const void* src, int64_t bytes, uint32_t fields) override {
@@ -1695,6 +1693,14 @@ class Engine final : public EngineBase {
     }
     mpm_status device_status() { return word_status(0, (int)I.size()); }
     mpm_status inst_status(int i) { return word_status(i, i + 1); }
+    // Waits for the stream; the status of instance i (its words come with the
+    // wait, the slow path only when one is set).
+    mpm_status sync_status(int i) {
+        launch_read_words(h_rb, d_err, d_ierr + i, st);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(st));
+        return (h_rb->err || h_rb->ierr) ? inst_status(i) : MPM_OK;
+    }
 
     mpm_status inst_statuses(int32_t* out, int n) override {
         if (!out || n < (int)I.size()) {
@@ -1723,14 +1729,14 @@ class Engine final : public EngineBase {
         // at least 4 particles per thread (256-thread CTAs), at most stat_blocks CTAs
         const int nb = (int)std::max<int64_t>(1, std::min<int64_t>(stat_blocks, (x.np + 4 * 256 - 1) / (4 * 256)));
         launch_stats<R>(d_inst + i, ps[cur], x.pbase, x.np, mu, K, x.p.rho_phys, x.p.cp, x.p.Tamb, d_stat_part, nb,
-                        d_stat_out, st);
-        double v[kStatSlots];
-        unsigned long long ctr[4];
-        double fsum[2];
-        CK(cudaMemcpyAsync(v, d_stat_out, sizeof(v), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(ctr, d_ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(fsum, d_ctr + 4, sizeof(fsum), cudaMemcpyDeviceToHost, st));
+                        h_rb, d_ctr, d_err, d_ierr + i, st);
+        CK(cudaGetLastError());
         CK(cudaStreamSynchronize(st));
+        const ReadBack rb = *h_rb;
+        const double* v = rb.stat;
+        const unsigned long long* ctr = rb.ctr;
+        double fsum[2];
+        std::memcpy(fsum, rb.ctr + 4, sizeof(fsum));
         // a NaN or Inf that never reached the positions (a temperature, stress or
         // plastic strain of a live particle) shows in the FP64 sums: it marks the
         // instance's word too (byte 0)
@@ -1771,7 +1777,7 @@ class Engine final : public EngineBase {
         out->contact_work = fsum[0];
         out->contact_force = fsum[1];
         out->n_asb_heated = (int64_t)ctr[3];
-        return inst_status(i);
+        return (finite && !rb.err && !rb.ierr) ? MPM_OK : inst_status(i);
     }
 
     // ---------------------------------------------------------------- misc

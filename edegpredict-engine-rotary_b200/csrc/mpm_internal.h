@@ -61,6 +61,15 @@ struct RelayoutMap {
 
 // Number of stats accumulators (see k_stats).
 constexpr int kStatSlots = 32;
+// 64-bit counters of a handle: four counts, then two FP64 sums.
+constexpr int kCounters = 6;
+// What a metrics or status read brings back, in pinned host memory that the
+// kernels write (valid after a synchronisation of their stream).
+struct ReadBack {
+    double stat[kStatSlots];
+    unsigned long long ctr[kCounters];
+    int err, ierr;   // the handle's error word and the instance's
+};
 
 // One heat-conduction diffusion step on grid buffer b of every instance that
 // conducts heat (node temperatures into Inst::tn).
@@ -143,7 +152,10 @@ void launch_ws_step(const Inst<R>* insts, const std::vector<int64_t>& np, const 
 
 template <typename R>
 void launch_stats(const Inst<R>* inst_dev, const PState<R>& ps, int64_t pbase, int64_t n, double mu, double K,
-                  double rho, double cp, double Tamb, double* partial, int nblocks, double* out, cudaStream_t st);
+                  double rho, double cp, double Tamb, double* partial, int nblocks, ReadBack* out,
+                  const unsigned long long* ctr, const int* err, const int* ierr, cudaStream_t st);
+// The error words alone.
+void launch_read_words(ReadBack* out, const int* err, const int* ierr, cudaStream_t st);
 
 // Copies particles [old_pbase, old_pbase + np) of every instance of `map`
 // (sorted by new_pbase) from src to [new_pbase, ...) of dst; total = slots of
