@@ -220,110 +220,90 @@ __global__ void k_bin_count(const Inst<R>* insts, int n_inst, PState<R> ps, cons
     rank[pi] = atomicAdd(&count[kk], 1);
 }
 
-// Position in its bin of the particle of cell c (0..63) with rank r among
-// that cell's particles; cs points at the bin's 65 cell offsets in the new
-// layout (cell q holds cs[q+1] - cs[q] particles, n = cs[64] - cs[0]).
-// The bin is a table of 64 columns, column c for cell c: with R = n / 64
-// full rows, particle (c, r < R) sits at r*64 + c.  The particles of cells
-// holding more than R (the overflow, in cell then rank order) fill first
-// the holes the smaller cells leave in the full rows (row m..R-1 of a cell
-// with m < R particles, in cell then row order), then the tail [64R, n).
-// A warp of the step kernel takes 32 consecutive positions: mostly 32
-// distinct cells of one half of the bin (x, y and two z layers), which is
-// what makes its velocity-tile gathers and node-tile adds conflict-free,
-// and a 256-particle pass holds at most four particles of a cell outside
-// the overflow.
-__device__ __forceinline__ int64_t column_slot(const int32_t* __restrict__ cs, int c, int r) {
-    const int n = cs[kCellsPerBin] - cs[0];
-    const int R = n / kCellsPerBin;
-    if (r < R) return (int64_t)r * kCellsPerBin + c;
-    int k = r - R;   // k-th overflow particle of the bin
-    for (int q = 0; q < c; ++q) {
-        const int m = cs[q + 1] - cs[q];
-        if (m > R) k += m - R;
-    }
-    for (int q = 0; q < kCellsPerBin; ++q) {
-        const int m = cs[q + 1] - cs[q];
-        const int holes = m < R ? R - m : 0;
-        if (k < holes) return (int64_t)(m + k) * kCellsPerBin + q;
-        k -= holes;
-    }
-    return (int64_t)R * kCellsPerBin + k;
-}
-
-// Destination slot of source slot pi in the new layout (-1: an unused slot).
+// The re-bin's move, in three launches so that the writes are coalesced: the
+// first files every source slot under its cell, the second orders the
+// particles of each bin and records for every destination slot its source
+// (perm[d] = pi), the third runs one thread per destination slot and copies
+// the particle from its source, which lies in the same bin's window of the
+// old layout (read through L2) -- a scatter by source slot wrote every 16-,
+// 4- and 1-byte field to a permuted slot and moved about twice the bytes
+// through DRAM.
+//
+// Filing: cell-major, in the atomics' arrival order (k_bin_count's rank):
+// perm[q] = the source, perm[np + q] = its upload position (read here, where
+// it is coalesced).  INACTIVE particles go to their final slot, after the
+// bins.
 template <typename R>
-__device__ __forceinline__ int64_t bin_dest(const Inst<R>& P, int ii, int64_t pi, const int32_t* key,
-                                            const int32_t* rank, const int32_t* offset, const int32_t* key_base,
-                                            const int32_t* newbin) {
-    if (pi >= P.pbase + P.np) return -1;
-    const int32_t kk = key[pi];
-    if (kk - key_base[ii] >= P.nbins * kCellsPerBin) return offset[kk] + rank[pi];  // INACTIVE: after the bins
-    const int32_t fk = key_base[ii] + newbin[pi] * kCellsPerBin;
-    return offset[fk] + column_slot(offset + fk, kk - fk, rank[pi]);
-}
-
-// The re-bin's move, in two launches so that the writes are coalesced: the
-// first records for every destination slot its source (perm[d] = pi), the
-// second runs one thread per destination slot and copies the particle from
-// its source, which lies in the same bin's window of the old layout (read
-// through L2) -- a scatter by source slot wrote every 16-, 4- and 1-byte field
-// to a permuted slot and moved about twice the bytes through DRAM.
-template <typename R>
-// perm[d] = the source slot of destination slot d, perm[np + d] = that
-// source's upload position (the order k_bin_order sorts by, read here where
-// it is coalesced).
 __global__ void k_bin_perm(const Inst<R>* insts, int n_inst, const int32_t* key, const int32_t* rank,
-                           const int32_t* offset, const int32_t* key_base, const int32_t* newbin,
-                           const int32_t* orig, int32_t* perm, int64_t np) {
+                           const int32_t* offset, const int32_t* orig, int32_t* perm, int64_t np) {
     const int64_t pi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pi >= np) return;
-    const int ii = find_inst(insts, n_inst, pi);
-    const int64_t d = bin_dest(insts[ii], ii, pi, key, rank, offset, key_base, newbin);
-    if (d >= 0) {
-        perm[d] = (int32_t)pi;
-        perm[np + d] = orig[pi];
-    }
+    const Inst<R>& P = insts[find_inst(insts, n_inst, pi)];
+    if (pi >= P.pbase + P.np) return;   // unused slot of the instance
+    const int64_t q = offset[key[pi]] + rank[pi];
+    perm[q] = (int32_t)pi;
+    perm[np + q] = orig[pi];
 }
 
-// The ranks of k_bin_count follow the atomics' arrival order.  One CTA per
-// bin of the bin table puts each cell's particles in the order of their
-// upload positions (orig): thread c takes the destinations of cell c (rank
-// order) and hands them the cell's sources sorted by orig.  The layout -- and
-// with it the order of every sum the step kernel forms -- then depends on the
-// particles' positions and upload order alone, not on the thread schedule or
-// the layout before (so re-binning a freshly binned state changes nothing).
+// The order of a bin's slots, one CTA per bin of the bin table, thread c its
+// cell c.  Each cell's particles are put in the order of their upload
+// positions, so that the layout -- and with it the order of every sum the step
+// kernel forms -- depends on the particles' positions and upload order alone,
+// not on the thread schedule or the layout before (re-binning a freshly binned
+// state changes nothing).  The slots go by rows: row r holds the r-th particle
+// of every cell that has more than r, in cell order; particle (c, r) sits at
+// sum over cells q < c of min(m_q, r + 1) plus over q >= c of min(m_q, r).  A
+// warp of the step kernel takes 32 consecutive slots: distinct cells wherever
+// a row is at least 32 wide, consecutive ones mostly, which is what makes its
+// velocity-tile gathers and node-tile adds conflict-free.  (Full rows of 64
+// columns with the surplus of fuller cells filled into the holes of emptier
+// ones put runs of one cell into a warp in bins at the workpiece's faces and
+// at 5 particles per cell, which then took several turns to scatter.)
 // Cells of up to kOrderLocal particles sort in registers and local memory; a
-// larger one (a cell packed several times over its particles per cell) takes
-// a selection sort through global memory.
+// bin with a larger one (a cell packed several times over its particles per
+// cell) takes selection sorts through global memory.
 constexpr int kOrderLocal = 48;
-
-__device__ __forceinline__ int64_t order_dest(const int32_t* cs, int c, int r, int64_t b0) {
-    return b0 + column_slot(cs, c, r);
-}
 
 __global__ void __launch_bounds__(kCellsPerBin) k_bin_order(const int32_t* __restrict__ bin_key,
                                                             const int32_t* __restrict__ offset, int32_t* perm,
                                                             int64_t np) {
-    const int32_t* __restrict__ okey = perm + np;   // upload position of each destination's source
     __shared__ int32_t cs[kCellsPerBin + 1];
+    __shared__ unsigned long long row[kCellsPerBin];   // cells with more than r particles
+    __shared__ int32_t start[kCellsPerBin];            // first slot of row r
     const int32_t fk = bin_key[blockIdx.x];
     const int c = threadIdx.x;
     cs[c] = offset[fk + c];
     if (c == 0) cs[kCellsPerBin] = offset[fk + kCellsPerBin];
     __syncthreads();
-    const int m = cs[c + 1] - cs[c];
-    if (m <= 1) return;
-    const int64_t b0 = cs[0];
-    if (m <= kOrderLocal) {
-        int32_t src[kOrderLocal], key[kOrderLocal];
-        int64_t dst[kOrderLocal];
-        for (int r = 0; r < m; ++r) {
-            dst[r] = order_dest(cs, c, r, b0);
-            src[r] = perm[dst[r]];
-            key[r] = okey[dst[r]];
+    if (cs[kCellsPerBin] == cs[0]) return;
+    {
+        unsigned long long m = 0ull;
+        int32_t before = 0;
+        for (int q = 0; q < kCellsPerBin; ++q) {
+            const int32_t n = cs[q + 1] - cs[q];
+            before += min(n, c);
+            if (n > c) m |= 1ull << q;
         }
-        // insertion sort by orig (distinct within an instance)
+        row[c] = m;
+        start[c] = before;
+    }
+    const int32_t m = cs[c + 1] - cs[c];
+    const int64_t b0 = cs[0], src0 = cs[c];
+    auto slot = [&](int r) -> int64_t {
+        if (r < kCellsPerBin) return b0 + start[r] + __popcll(row[r] & ((1ull << c) - 1ull));
+        int64_t s = b0;
+        for (int q = 0; q < kCellsPerBin; ++q) s += min(cs[q + 1] - cs[q], q < c ? r + 1 : r);
+        return s;
+    };
+    int32_t* okey = perm + np;   // upload positions
+    if (!__syncthreads_or(m > kOrderLocal)) {
+        int32_t src[kOrderLocal], key[kOrderLocal];
+        for (int r = 0; r < m; ++r) {
+            src[r] = perm[src0 + r];
+            key[r] = okey[src0 + r];
+        }
+        __syncthreads();   // every source is read before the slots, the same entries, are written
+        // insertion sort by upload position (distinct within an instance)
         for (int r = 1; r < m; ++r) {
             const int32_t v = src[r], k = key[r];
             int q = r - 1;
@@ -335,32 +315,32 @@ __global__ void __launch_bounds__(kCellsPerBin) k_bin_order(const int32_t* __res
             src[q + 1] = v;
             key[q + 1] = k;
         }
-        for (int r = 0; r < m; ++r) perm[dst[r]] = src[r];
-    } else {
-        // selection sort in place: rank r takes the smallest orig among ranks r..m-1
-        for (int r = 0; r < m - 1; ++r) {
-            const int64_t dr = order_dest(cs, c, r, b0);
-            int64_t best = dr;
-            int32_t bv = perm[dr], bk = okey[dr];
-            for (int q = r + 1; q < m; ++q) {
-                const int64_t dq = order_dest(cs, c, q, b0);
-                const int32_t v = perm[dq], k = okey[dq];
-                if (k < bk) { bv = v; bk = k; best = dq; }
-            }
-            if (best != dr) {
-                perm[best] = perm[dr];
-                perm[np + best] = okey[dr];
-                perm[dr] = bv;
-                perm[np + dr] = bk;
-            }
+        for (int r = 0; r < m; ++r) perm[slot(r)] = src[r];
+        return;
+    }
+    // selection sort in place, then through the upload positions' place into the slots
+    for (int r = 0; r < m - 1; ++r) {
+        int best = r;
+        for (int q = r + 1; q < m; ++q)
+            if (okey[src0 + q] < okey[src0 + best]) best = q;
+        if (best != r) {
+            const int32_t v = perm[src0 + r], k = okey[src0 + r];
+            perm[src0 + r] = perm[src0 + best];
+            okey[src0 + r] = okey[src0 + best];
+            perm[src0 + best] = v;
+            okey[src0 + best] = k;
         }
     }
+    __syncthreads();
+    for (int r = 0; r < m; ++r) okey[slot(r)] = perm[src0 + r];
+    __syncthreads();
+    for (int64_t q = b0 + c; q < cs[kCellsPerBin]; q += kCellsPerBin) perm[q] = okey[q];
 }
 
 template <typename R>
 __global__ void k_bin_gather(PState<R> src, PState<R> dst, const Inst<R>* insts, int n_inst, const int32_t* key,
                              const int32_t* key_base, const int32_t* newbin, const int32_t* perm, bool initial,
-                             const double* pos_scratch, bool has_K, int64_t np) {
+                             const double* pos_scratch, bool has_K, bool mid_call, int64_t np) {
     const int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= np) return;
     const int64_t pi = perm[d];
@@ -393,8 +373,16 @@ __global__ void k_bin_gather(PState<R> src, PState<R> dst, const Inst<R>* insts,
     dst.skey[d] = key[pi] - key_base[ii];
 #pragma unroll
     for (int q = 1; q < 6; ++q) dst.A[q][d] = src.A[q][pi];
+    // Inside a fused call v, C and the strain rate of an ACTIVE particle live in
+    // the step kernel's registers from each G2P to its P2G: what memory holds is
+    // of an earlier call, and whatever takes the particle out of the cycle (the
+    // last G2P of the call, a kill, a chip) writes them.  384 instead of 512
+    // bytes moved: 33.5 M particles 2.1 instead of 2.7 ms.
+    const uint8_t st = src.status[pi];
+    if (!(mid_call && st == ST_ACTIVE)) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) dst.B[q][d] = src.B[q][pi];
+        for (int q = 0; q < 4; ++q) dst.B[q][d] = src.B[q][pi];
+    }
     dst.S[0][d] = src.S[0][pi];
     dst.S[1][d] = src.S[1][pi];
     if (has_K) {
@@ -402,7 +390,7 @@ __global__ void k_bin_gather(PState<R> src, PState<R> dst, const Inst<R>* insts,
         dst.K[1][d] = src.K[1][pi];
     }
     dst.sres[d] = src.sres[pi];
-    dst.status[d] = src.status[pi];
+    dst.status[d] = st;
     dst.asb[d] = src.asb[pi];
     dst.id[d] = src.id[pi];
     dst.orig[d] = src.orig[pi];
@@ -991,15 +979,15 @@ void launch_bin_count(const Inst<R>* insts, int n_inst, const PState<R>& ps, con
 template <typename R>
 void launch_bin_scatter(const PState<R>& src, const PState<R>& dst, const Inst<R>* insts, int n_inst,
                         const int32_t* key, const int32_t* rank, const int32_t* offset, const int32_t* key_base,
-                        const int32_t* newbin, bool initial, const double* pos_scratch, bool has_K, int64_t np,
-                        int32_t* perm, const int32_t* bin_key, int nbins_total, cudaStream_t st) {
+                        const int32_t* newbin, bool initial, const double* pos_scratch, bool has_K, bool mid_call,
+                        int64_t np, int32_t* perm, const int32_t* bin_key, int nbins_total, cudaStream_t st) {
     if (np <= 0) return;
     const int blocks = (int)((np + kT - 1) / kT);
     cudaMemsetAsync(perm, 0xff, sizeof(int32_t) * np, st);
-    k_bin_perm<R><<<blocks, kT, 0, st>>>(insts, n_inst, key, rank, offset, key_base, newbin, src.orig, perm, np);
+    k_bin_perm<R><<<blocks, kT, 0, st>>>(insts, n_inst, key, rank, offset, src.orig, perm, np);
     if (nbins_total > 0) k_bin_order<<<nbins_total, kCellsPerBin, 0, st>>>(bin_key, offset, perm, np);
     k_bin_gather<R><<<blocks, kT, 0, st>>>(src, dst, insts, n_inst, key, key_base, newbin, perm, initial,
-                                           pos_scratch, has_K, np);
+                                           pos_scratch, has_K, mid_call, np);
     launch_counter() += nbins_total > 0 ? 3 : 2;
 }
 
@@ -1192,7 +1180,7 @@ void launch_heat_diffuse(const Inst<R>* insts, int n_inst, int b, int64_t total,
                                       int32_t*, int32_t*, int32_t*, int32_t*, int64_t, int, int, bool, cudaStream_t); \
     template void launch_bin_scatter<R>(const PState<R>&, const PState<R>&, const Inst<R>*, int, const int32_t*,    \
                                         const int32_t*, const int32_t*, const int32_t*, const int32_t*, bool,       \
-                                        const double*, bool, int64_t, int32_t*, const int32_t*, int, cudaStream_t);  \
+                                        const double*, bool, bool, int64_t, int32_t*, const int32_t*, int, cudaStream_t);  \
     template void launch_import<R>(const DevSoA&, int64_t, double, double, double, double, double, const PState<R>&, \
                                    int64_t, double*, cudaStream_t);                                                  \
     template void launch_gen<R>(const Inst<R>&, const int32_t*, const int32_t*, int, uint64_t, uint32_t, int, double, \

@@ -807,7 +807,7 @@ class Engine final : public EngineBase {
                             cap_total, det ? 0 : -1, sort_every, det, st);
         exclusive_scan(d_count, d_offset, nkeys, d_scan_tmp, st);
         launch_bin_scatter<R>(ps[cur], ps[cur ^ 1], d_inst, (int)I.size(), d_key, d_rank, d_offset, d_key_base,
-                              d_newbin, true, d_pos, has_K, cap_total, d_perm, d_bin_key, max_work, st);
+                              d_newbin, true, d_pos, has_K, false, cap_total, d_perm, d_bin_key, max_work, st);
         build_work(d_offset, d_bin_key, d_bin_inst, d_bin_local, d_inst_pbase, max_work, d_flag, d_flag_scan,
                    d_scan_tmp, d_work, d_nwork, st);
         cur ^= 1;
@@ -1320,7 +1320,7 @@ class Engine final : public EngineBase {
             }
             if (any && !det)
                 for (size_t i = 0; i < I.size(); ++i) last[i] = k;
-            return any ? rebin_regular(det ? k : -1) : MPM_OK;
+            return any ? rebin_regular(det ? k : -1, fused) : MPM_OK;
         };
         const int cps = ctas_per_sm;
         int xk = 0, heat = 0;
@@ -1587,7 +1587,7 @@ class Engine final : public EngineBase {
             for (auto& x : I) x.since = 0;
             cudaEventRecord(e0, st);
             if ((s = step(n, dts)) != MPM_OK) return s;
-            if ((s = rebin_regular(-1)) != MPM_OK) return s;
+            if ((s = rebin_regular(-1, false)) != MPM_OK) return s;
             for (auto& x : I) x.since = 0;
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess) {
@@ -1635,8 +1635,9 @@ class Engine final : public EngineBase {
 
     // The re-bin at point kpt of a step call: the instances whose re-bin
     // phase falls on kpt are binned from their positions, the others keep
-    // their layout (kpt < 0: every instance is re-binned).
-    mpm_status rebin_regular(int kpt) {
+    // their layout (kpt < 0: every instance is re-binned).  mid_call: between two
+    // launches of a fused step call.
+    mpm_status rebin_regular(int kpt, bool mid_call) {
         Range nvtx_range("mpm.rebin");
         // positions are bin-local (no instance is fresh here)
         CK(cudaMemsetAsync(d_count, 0, 4 * (nkeys + 1), st));
@@ -1645,7 +1646,7 @@ class Engine final : public EngineBase {
                             d_newbin, cap_total, kpt, sort_every, false, st);
         exclusive_scan(d_count, d_offset, nkeys, d_scan_tmp, st);
         launch_bin_scatter<R>(ps[cur], ps[cur ^ 1], d_inst, (int)I.size(), d_key, d_rank, d_offset, d_key_base,
-                              d_newbin, false, d_pos, has_K, cap_total, d_perm, d_bin_key, max_work, st);
+                              d_newbin, false, d_pos, has_K, mid_call, cap_total, d_perm, d_bin_key, max_work, st);
         build_work(d_offset, d_bin_key, d_bin_inst, d_bin_local, d_inst_pbase, max_work, d_flag, d_flag_scan,
                    d_scan_tmp, d_work, d_nwork, st);
         cur ^= 1;

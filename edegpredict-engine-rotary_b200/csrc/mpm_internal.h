@@ -97,11 +97,12 @@ void launch_bin_count(const Inst<R>* insts, int n_inst, const PState<R>& ps, con
 
 // The re-bin's move: every particle to its slot in the new layout, each
 // cell's particles in the order of their old slots (bin_key: the first key
-// of each of the nbins_total bins of the bin table).
+// of each of the nbins_total bins of the bin table).  mid_call: inside a fused
+// step call, where B of ACTIVE particles is dead and stays behind.
 template <typename R>
 void launch_bin_scatter(const PState<R>& src, const PState<R>& dst, const Inst<R>* insts, int n_inst,
                         const int32_t* key, const int32_t* rank, const int32_t* offset, const int32_t* key_base,
-                        const int32_t* newbin, bool initial, const double* pos_scratch, bool has_K, int64_t np,
+                        const int32_t* newbin, bool initial, const double* pos_scratch, bool has_K, bool mid_call, int64_t np,
                         int32_t* perm, const int32_t* bin_key, int nbins_total, cudaStream_t st);
 // (perm holds 2 np int32: the permutation, then its sources' upload positions)
 

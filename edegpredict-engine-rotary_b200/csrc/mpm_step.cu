@@ -1108,13 +1108,11 @@ template <typename R> struct PairCoef {
 // Adds the particles of a warp (one per lane; staged: the lane has one whose
 // stencil lies in the tile, base cell (bx, by, bz)) to the warp's own node
 // tile: per stencil offset a load, two FMAs a pair and a store, phases
-// separated by __syncwarp.  A turn takes lanes with distinct cells of one half
-// of the bin (z 0-1 or 2-3): within a phase they address distinct nodes, so
-// plain load-add-stores do not collide, and two offsets whose k differs by 2
-// cannot meet at a node either, so k = 0 and k = 2 share a phase.  The re-bin's
-// column layout makes almost every warp one turn; lanes that share a cell or
-// left the half (moved since the re-bin, or of an overfull cell) wait for a
-// later one, lowest lane first, so the sums have a fixed order.
+// separated by __syncwarp.  A turn takes lanes with distinct cells: within a
+// phase they address distinct nodes, so plain load-add-stores do not collide.
+// The re-bin's rows make almost every warp one turn; lanes that share a cell
+// (moved since the re-bin, or rows narrower than a warp) wait for a later one,
+// lowest lane first, so the sums have a fixed order.
 // Against the staging of payloads in passes that a thread pair per cell then
 // summed (two CTA barriers a pass, 54 accumulators a thread): 225 M warp
 // instructions instead of 261 M on 4.2 M particles, 3.32 instead of 3.77 ms
@@ -1141,11 +1139,9 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
     const PairCoef<R> B(w, dw, mk2(p.Q[1], p.Q[2]), mk2(p.Rm[3], p.Rm[6]), mk2(p.Rm[4], p.Rm[7]),
                         mk2(p.Rm[5], p.Rm[8]), mk2(p.S[3], p.S[6]), mk2(p.S[4], p.S[7]), mk2(p.S[5], p.S[8]));
     do {
-        const int half = __shfl_sync(0xffffffffu, bz >> 1, __ffs((int)todo) - 1);
-        const bool in = ((todo >> lane) & 1u) && (bz >> 1) == half;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
         bool mine = false;
-        if (in) mine = (__ffs((int)__match_any_sync(m, bx + kBin * (by + kBin * bz))) - 1) == lane;
+        if ((todo >> lane) & 1u)
+            mine = (__ffs((int)__match_any_sync(todo, bx + kBin * (by + kBin * bz))) - 1) == lane;
         todo &= ~__ballot_sync(0xffffffffu, mine);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -1164,14 +1160,11 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
                 const P2 b = fma2(w[1][j], PB[k], fma2(QB, w[2][k], mk2(o.z, o.w)));
                 return mk4<R>(lo2(a), hi2(a), lo2(b), hi2(b));
             };
-            __syncwarp();
-            if (mine) {
-                const V4<R> o0 = n[0], o2 = n[2 * kLayer];
-                n[0] = added(o0, 0);
-                n[2 * kLayer] = added(o2, 2);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                __syncwarp();
+                if (mine) n[kLayer * k] = added(n[kLayer * k], k);
             }
-            __syncwarp();
-            if (mine) n[kLayer] = added(n[kLayer], 1);
         }
     }
     __syncwarp();
@@ -1787,13 +1780,12 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
             for (int nidx = tid; nidx < kTileNodes; nidx += kNT) {
                 const int X = nidx % kTile, Y = (nidx / kTile) % kTile, Z = nidx / (kTile * kTile);
                 const int t = sidx(X, Y, Z), tt = tidx(X, Y, Z);
-                // (warps 0 and 2 hold the lower half's cells, 1 and 3 the upper's)
-                const V4<R> e0 = Sm.acc[0][t], e1 = Sm.acc[2][t], e2 = Sm.acc[1][t], e3 = Sm.acc[3][t];
+                const V4<R> e0 = Sm.acc[0][t], e1 = Sm.acc[1][t], e2 = Sm.acc[2][t], e3 = Sm.acc[3][t];
                 const V4<R> node = mk4<R>((e0.x + e1.x) + (e2.x + e3.x), (e0.y + e1.y) + (e2.y + e3.y),
                                           (e0.z + e1.z) + (e2.z + e3.z), (e0.w + e1.w) + (e2.w + e3.w));
                 R mT = R(0);
                 if (EXT)
-                    mT = (Sm.nT[0][tt] + Sm.nT[EXT ? 2 : 0][tt]) + (Sm.nT[EXT ? 1 : 0][tt] + Sm.nT[EXT ? 3 : 0][tt]);
+                    mT = (Sm.nT[0][tt] + Sm.nT[EXT ? 1 : 0][tt]) + (Sm.nT[EXT ? 2 : 0][tt] + Sm.nT[EXT ? 3 : 0][tt]);
 #pragma unroll
                 for (int q = 0; q < kWarps; ++q) {
                     Sm.acc[q][t] = mk4<R>(R(0), R(0), R(0), R(0));
