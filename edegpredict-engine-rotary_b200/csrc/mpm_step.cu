@@ -1042,6 +1042,11 @@ template <typename R> constexpr int kMinCtas = sizeof(R) == 4 ? MPMB_MIN_CTAS : 
 // cycles per issued instruction, with the stage 0.2 of 6.6.
 constexpr int kStageGroups = 7;
 
+// Pairs of a tile's nodes: the 16 lanes of a half warp (x and y 0-3 of one z)
+// read 16 distinct 8-byte bank pairs.
+constexpr int kPairSlots = 72 * kTile;
+__device__ __forceinline__ int pidx(int x, int y, int z) { return x + 12 * y + 72 * z; }
+
 // EXT: the kernel variant with the extensions (adiabatic shear heating, heat
 // conduction, voxel contact), which adds the T m node sums (nT) and the node
 // temperature tile with its m > 1e-18 mask (ttile).
@@ -1054,7 +1059,8 @@ template <typename R, bool EXT> struct StepSmem {
     V4<R> acc[kWarps][kTileSlots];
     V4<R> stage[sizeof(R) == 4 ? kStageGroups : 1][sizeof(R) == 4 ? kNT : 1];
     R nT[EXT ? kWarps : 1][EXT ? kPlane : 1];   // T m (tidx layout), the same way
-    R ttile[EXT ? 2 : 1][EXT ? kPlane : 1];     // node temperatures and their m > 1e-18 mask
+    // node temperatures and their m > 1e-18 mask (0 or 1) as pairs (pidx)
+    P2T<R> ttile[EXT ? kPairSlots : 1];
     // the work item's tool poses at the G2P step (x, y, z) and at the P2G step:
     // read where used (volatile), so that no thread holds them in registers
     // across the particle loop
@@ -1125,6 +1131,8 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
     if (todo == 0u) return;
     const Stencil sl(bx, by, bz);
     V4<R>* __restrict__ tile = Sm.acc[wid];
+    R* __restrict__ nt = Sm.nT[EXT ? wid : 0] + (EXT ? tidx(bx, by, bz) : 0);
+    const R mT = EXT ? pm * p.T : R(0);
     P2 w[3][3];
     R w1[3][3], dw[3][3];
 #pragma unroll
@@ -1155,6 +1163,7 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
         for (int j = 0; j < 3; ++j) {
             const P2 QA = mul2(w[0][i], A.Cy[j]), QB = mul2(w[0][i], B.Cy[j]);
             V4<R>* n = tile + sl.at(i, j) + kRow * j;
+            const R mxy = EXT ? mT * w1[0][i] * w1[1][j] : R(0);
             auto added = [&](const V4<R>& o, int k) {
                 const P2 a = fma2(w[1][j], PA[k], fma2(QA, w[2][k], mk2(o.x, o.y)));
                 const P2 b = fma2(w[1][j], PB[k], fma2(QB, w[2][k], mk2(o.z, o.w)));
@@ -1163,28 +1172,15 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 __syncwarp();
-                if (mine) n[kLayer * k] = added(n[kLayer * k], k);
+                if (mine) {
+                    n[kLayer * k] = added(n[kLayer * k], k);
+                    // heat conduction: the T m channel, w m T
+                    if (EXT && heat) nt[i + kSY * j + kSZ * k] = fma(mxy, w1[2][k], nt[i + kSY * j + kSZ * k]);
+                }
             }
         }
     }
     __syncwarp();
-    if (EXT && heat) {
-        // heat conduction: the T m channel, w m T
-        R* __restrict__ t = Sm.nT[EXT ? wid : 0] + tidx(bx, by, bz);
-        const R mT = pm * p.T;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const R mxy = mT * w1[0][i] * w1[1][j];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    __syncwarp();
-                    if (mine) t[i + kSY * j + kSZ * k] = fma(mxy, w1[2][k], t[i + kSY * j + kSZ * k]);
-                }
-            }
-        __syncwarp();
-    }
     } while (todo);
 }
 
@@ -1325,15 +1321,14 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
             for (int nidx = tid; nidx < kTileNodes; nidx += kNT) {
                 const int lx = nidx % kTile, ly = (nidx / kTile) % kTile, lz = nidx / (kTile * kTile);
                 const NV<R> nv = node_vel_inl(P, Sm.raw[nidx], g0x + lx, g0y + ly, g0z + lz, pose[0], pose[2]);
-                const int t = tidx(lx, ly, lz);
                 Sm.vel[sidx(lx, ly, lz)] = mk4<R>(nv.x, nv.y, nv.z, nv.z);
                 if (EXT && P.heat_on) {
                     // node temperatures after the diffusion step, for the nodes the
                     // temperature gather counts (m > 1e-18, inside the domain)
                     const int gx = g0x + lx, gy = g0y + ly, gz = g0z + lz;
                     const bool use = Sm.raw[nidx].x > R(1e-18) && gx < P.nx && gy < P.ny && gz < P.nz;
-                    Sm.ttile[0][t] = use ? P.tn[gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz)] : R(0);
-                    Sm.ttile[1][t] = use ? R(1) : R(0);
+                    Sm.ttile[EXT ? pidx(lx, ly, lz) : 0] =
+                        mk2(use ? P.tn[gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz)] : R(0), use ? R(1) : R(0));
                 }
             }
         }
@@ -1400,20 +1395,19 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                             if (__builtin_expect(b[0] >= 0 && b[0] < kBin && b[1] >= 0 && b[1] < kBin && b[2] >= 0 && b[2] < kBin, 1)) {
                                 gather_tile<R>(Sm.vel, Stencil(b[0], b[1], b[2]), w, dw, v, M, L);
                                 if (EXT && P.heat_on) {
-                                    const int tb = tidx(b[0], b[1], b[2]);
+                                    const P2T<R>* tb = Sm.ttile + pidx(b[0], b[1], b[2]);
+                                    P2T<R> sum = dup2(R(0));   // (sum w T, sum w) over the counted nodes
 #pragma unroll
                                     for (int k = 0; k < 3; ++k)
 #pragma unroll
                                         for (int j = 0; j < 3; ++j) {
                                             const R wjk = w[1][j] * w[2][k];
 #pragma unroll
-                                            for (int i = 0; i < 3; ++i) {
-                                                const int q = tb + i + kSY * j + kSZ * k;
-                                                const R ww = w[0][i] * wjk;
-                                                tsum.ts = fma(ww, Sm.ttile[0][q], tsum.ts);
-                                                tsum.ws = fma(ww, Sm.ttile[1][q], tsum.ws);
-                                            }
+                                            for (int i = 0; i < 3; ++i)
+                                                sum = fma2(dup2(w[0][i] * wjk), tb[EXT ? pidx(i, j, k) : 0], sum);
                                         }
+                                    tsum.ts = lo2(sum);
+                                    tsum.ws = hi2(sum);
                                 }
                             } else {
                                 const GatherOut<R> go = gather_global<R>(P, gr, g0x, g0y, g0z, xi[0], xi[1], xi[2],
