@@ -237,7 +237,8 @@ __device__ __forceinline__ NV<R> node_vel_inl(const Inst<R>& P, const V4<R> g, i
     NV<R> out{R(0), R(0), R(0)};
     if (!(m > (R)P.mthr)) return out;
     R vx = g.y / m, vy = g.z / m, vz = (g.w + m * (R)(P.grav * P.dt)) / m;
-    if (P.fix_thick > 0.0) {
+    // (the exact ratio only near or inside the layer: a product decides the rest)
+    if (P.fix_thick > 0.0 && dm((double)gz, P.dx) <= P.fix_thick * (1.0 + 1e-6) + 1e-6 * fabs(P.oz)) {
         const double zr = ds(node_coord(gz, P.dx, P.oz), P.oz) / P.fix_thick;
         if (zr <= 1.0) {
             if (gz == 0) {
@@ -283,12 +284,6 @@ __device__ __forceinline__ NV<R> node_vel_inl(const Inst<R>& P, const V4<R> g, i
     }
     out.x = vx; out.y = vy; out.z = vz;
     return out;
-}
-
-// Out-of-line copy for the slow-path gather (keeps its 27 node updates small).
-template <typename R>
-__device__ __noinline__ NV<R> node_vel(const Inst<R>& P, const V4<R> g, int gx, int gy, int gz, double pr0, double pr2) {
-    return node_vel_inl<R>(P, g, gx, gy, gz, pr0, pr2);
 }
 
 // ------------------------------------------------------------------ gather (G2P)
@@ -389,46 +384,48 @@ __device__ __forceinline__ void gather_tile(const V4<R>* vel, const Stencil& sl,
 }
 
 // Same sums for a particle whose stencil left its bin's tile: nodes are read
-// and updated straight from the grid (rare; the re-bin brings it back).  Out
-// of line, with its inputs and result by value, so that the hot path keeps
-// its arrays in registers.
+// and updated straight from the grid (rare; the re-bin brings it back).  The
+// lanes of the warp that are here update a node each (rank of n lanes; the
+// velocity and whether the node lies in the domain go to nv), then the
+// particle's lane sums them.  One lane updating its 27 nodes, tool distance in
+// FP64 and all, took about 20 us: as long as a bin, and the particles that
+// leave their bins are those at the tool, so a launch of 0.5 M particles
+// waited 35 us for its last bins.
+template <typename R>
+__device__ __noinline__ void far_nodes(const Inst<R>& P, const V4<R>* __restrict__ grid, int gx0, int gy0, int gz0,
+                                       double pr0, double pr2, V4<R>* nv, int rank, int n) {
+    for (int q = rank; q < 27; q += n) {
+        const int gx = gx0 + q / 9, gy = gy0 + (q / 3) % 3, gz = gz0 + q % 3;
+        const int64_t gi = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
+        const bool in = gx >= 0 && gx < P.nx && gy >= 0 && gy < P.ny && gz >= 0 && gz < P.nz &&
+                        MPMB_CHECK(gi >= 0 && gi < P.nn, kSiteGather, gi);
+        NV<R> v{R(0), R(0), R(0)};
+        if (in) v = node_vel_inl(P, grid[gi], gx, gy, gz, pr0, pr2);
+        nv[q] = mk4<R>(v.x, v.y, v.z, in ? R(1) : R(0));
+    }
+}
+
 template <typename R> struct GatherOut {
     R v[3], M[3][3], L[3][3];
 };
 
-template <typename R>
-__device__ __noinline__ GatherOut<R> gather_global(const Inst<R>& P, const V4<R>* __restrict__ grid, int g0x, int g0y,
-                                                   int g0z, R x0, R x1, R x2, double pr0, double pr2) {
+// The sums of a particle at offset (d0, d1, d2) from its base node.
+template <typename R> __device__ __noinline__ GatherOut<R> far_sum(const V4<R>* nv, R d0, R d1, R d2) {
     GatherOut<R> o;
     R w[3][3], dw[3][3];
-    int gb[3];
-    gb[0] = g0x + bspline(x0, w[0], dw[0]);
-    gb[1] = g0y + bspline(x1, w[1], dw[1]);
-    gb[2] = g0z + bspline(x2, w[2], dw[2]);
+    bspline_at(d0, w[0], dw[0]);
+    bspline_at(d1, w[1], dw[1]);
+    bspline_at(d2, w[2], dw[2]);
     for (int c = 0; c < 3; ++c) {
         o.v[c] = R(0);
         for (int b = 0; b < 3; ++b) { o.M[c][b] = R(0); o.L[c][b] = R(0); }
     }
-    // the 27 node loads first, all in flight together, then the node updates
-    V4<R> gv[27];
-    bool in[27];
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int gx = gb[0] + q / 9, gy = gb[1] + (q / 3) % 3, gz = gb[2] + q % 3;
-        const int64_t gi = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
-        in[q] = gx >= 0 && gx < P.nx && gy >= 0 && gy < P.ny && gz >= 0 && gz < P.nz &&
-                MPMB_CHECK(gi >= 0 && gi < P.nn, kSiteGather, gi);
-        gv[q] = in[q] ? grid[gi] : mk4<R>(R(0), R(0), R(0), R(0));
-    }
     for (int i = 0; i < 3; ++i) {
-        const int gx = gb[0] + i;
         for (int j = 0; j < 3; ++j) {
-            const int gy = gb[1] + j;
             for (int k = 0; k < 3; ++k) {
-                const int gz = gb[2] + k;
-                if (!in[i * 9 + j * 3 + k]) continue;
-                const NV<R> nv = node_vel(P, gv[i * 9 + j * 3 + k], gx, gy, gz, pr0, pr2);
-                const R vv[3] = {nv.x, nv.y, nv.z};
+                const V4<R> n = nv[i * 9 + j * 3 + k];
+                if (n.w == R(0)) continue;
+                const R vv[3] = {n.x, n.y, n.z};
                 const R ww = w[0][i] * w[1][j] * w[2][k];
                 const R g0 = dw[0][i] * w[1][j] * w[2][k], g1 = w[0][i] * dw[1][j] * w[2][k],
                         g2 = w[0][i] * w[1][j] * dw[2][k];
@@ -452,13 +449,6 @@ __device__ __noinline__ GatherOut<R> gather_global(const Inst<R>& P, const V4<R>
 // Momentum + impulse at node (i,j,k):
 //   p_a = w_ijk (Q_a + R_ax i + R_ay j + R_az k) + S_ax dwx wy wz + S_ay wx dwy wz + S_az wx wy dwz
 // with Q = m (v - dx C d), R = m dx C, S = -dt V J sigma / dx.  Separable in k.
-// Scatter of a particle whose stencil left its bin's tile: straight into the
-// grid with vector atomics (rare; out of line, inputs by value).
-template <typename R> struct ScatterIn {
-    R xi[3], Q[3], Rm[9], S[9];
-    int g0[3];
-};
-
 // Deterministic mode: channel ch of node gi gets v in fixed point (rounded to
 // a multiple of 1/esc_scale, clamped to +-4e18 units; integer adds commute, so
 // the escaped sums do not depend on the order of the particles).
@@ -472,76 +462,50 @@ template <typename R> __device__ __forceinline__ void esc_mark(const Inst<R>& P,
     P.esc_flag[gx / kBin + P.nbx * (gy / kBin + P.nby * (gz / kBin))] = 1;
 }
 
+// What a particle scatters: its offset from its base node after the move (cells),
+// Q = m (v - dx C d) + f_ext dt, R = m dx C and S = -dt V J sigma / dx
+// (row-major), T absolute (heat conduction).
+template <typename R> struct Payload {
+    R d[3], Q[3], Rm[9], S[9], T;
+};
+
+// Scatter of a particle whose stencil left its bin's tile, straight into the
+// grid (rare): lane q of the warp takes node q of the 27 (base node gx0, gy0,
+// gz0; p and m the same in every lane).  tw: the T m write buffer, with heat
+// conduction.
 template <typename R>
-__device__ __noinline__ void scatter_global(const Inst<R>& P, V4<R>* __restrict__ grid, const ScatterIn<R> in, R m) {
+__device__ __noinline__ void far_scatter(const Inst<R>& P, V4<R>* __restrict__ grid, R* __restrict__ tw, int gx0,
+                                         int gy0, int gz0, const Payload<R> in, R m, int lane) {
+    if (lane >= 27) return;
+    const int i = lane / 9, j = (lane / 3) % 3, k = lane % 3;
+    const int gx = gx0 + i, gy = gy0 + j, gz = gz0 + k;
+    if (gx < 0 || gx >= P.nx || gy < 0 || gy >= P.ny || gz < 0 || gz >= P.nz) return;
+    const int64_t gi = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
+    if (!MPMB_CHECK(gi >= 0 && gi < P.nn, kSiteScatter, gi)) return;
     R w[3][3], dw[3][3];
-    int gb[3];
-    for (int a = 0; a < 3; ++a) gb[a] = in.g0[a] + bspline(in.xi[a], w[a], dw[a]);
-    for (int i = 0; i < 3; ++i) {
-        const int gx = gb[0] + i;
-        if (gx < 0 || gx >= P.nx) continue;
-        for (int j = 0; j < 3; ++j) {
-            const int gy = gb[1] + j;
-            if (gy < 0 || gy >= P.ny) continue;
-            for (int k = 0; k < 3; ++k) {
-                const int gz = gb[2] + k;
-                if (gz < 0 || gz >= P.nz) continue;
-                const R ww = w[0][i] * w[1][j] * w[2][k];
-                const R g0 = dw[0][i] * w[1][j] * w[2][k], g1 = w[0][i] * dw[1][j] * w[2][k],
-                        g2 = w[0][i] * w[1][j] * dw[2][k];
-                R p[3];
-                for (int a = 0; a < 3; ++a)
-                    p[a] = ww * (in.Q[a] + in.Rm[a * 3] * R(i) + in.Rm[a * 3 + 1] * R(j) + in.Rm[a * 3 + 2] * R(k)) +
-                           in.S[a * 3] * g0 + in.S[a * 3 + 1] * g1 + in.S[a * 3 + 2] * g2;
-                const int64_t gi = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
-                if (!MPMB_CHECK(gi >= 0 && gi < P.nn, kSiteScatter, gi)) continue;
-                if (P.esc) {
-                    esc_add<R>(P, gi, 0, ww * m);
-                    esc_add<R>(P, gi, 1, p[0]);
-                    esc_add<R>(P, gi, 2, p[1]);
-                    esc_add<R>(P, gi, 3, p[2]);
-                    esc_mark<R>(P, gx, gy, gz);
-                } else {
-                    vec_atomic_add<R>(&grid[gi], ww * m, p[0], p[1], p[2]);
-                }
-            }
-        }
+    for (int a = 0; a < 3; ++a) bspline_at(in.d[a], w[a], dw[a]);
+    const R ww = w[0][i] * w[1][j] * w[2][k];
+    const R g0 = dw[0][i] * w[1][j] * w[2][k], g1 = w[0][i] * dw[1][j] * w[2][k], g2 = w[0][i] * w[1][j] * dw[2][k];
+    R p[3];
+    for (int a = 0; a < 3; ++a)
+        p[a] = ww * (in.Q[a] + in.Rm[a * 3] * R(i) + in.Rm[a * 3 + 1] * R(j) + in.Rm[a * 3 + 2] * R(k)) +
+               in.S[a * 3] * g0 + in.S[a * 3 + 1] * g1 + in.S[a * 3 + 2] * g2;
+    if (P.esc) {
+        esc_add<R>(P, gi, 0, ww * m);
+        esc_add<R>(P, gi, 1, p[0]);
+        esc_add<R>(P, gi, 2, p[1]);
+        esc_add<R>(P, gi, 3, p[2]);
+        if (tw) esc_add<R>(P, gi, 4, ww * (m * in.T));
+        esc_mark<R>(P, gx, gy, gz);
+    } else {
+        vec_atomic_add<R>(&grid[gi], ww * m, p[0], p[1], p[2]);
+        if (tw) atomicAdd(&tw[gi], ww * (m * in.T));
     }
 }
 
-// Heat conduction on the global paths (particles whose stencil left the bin
-// tile): the T m scatter into the write buffer, and the temperature gather
-// over the nodes with m > 1e-18 (sum of w T and of w), as the tile paths do.
-template <typename R>
-__device__ __noinline__ void scatter_T_global(const Inst<R>& P, R* __restrict__ tw, int g0x, int g0y, int g0z, R x0,
-                                              R x1, R x2, R mT) {
-    R w[3][3], dw[3][3];
-    int gb[3];
-    gb[0] = g0x + bspline(x0, w[0], dw[0]);
-    gb[1] = g0y + bspline(x1, w[1], dw[1]);
-    gb[2] = g0z + bspline(x2, w[2], dw[2]);
-    for (int i = 0; i < 3; ++i) {
-        const int gx = gb[0] + i;
-        if (gx < 0 || gx >= P.nx) continue;
-        for (int j = 0; j < 3; ++j) {
-            const int gy = gb[1] + j;
-            if (gy < 0 || gy >= P.ny) continue;
-            for (int k = 0; k < 3; ++k) {
-                const int gz = gb[2] + k;
-                if (gz < 0 || gz >= P.nz) continue;
-                const int64_t gi = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
-                if (!MPMB_CHECK(gi >= 0 && gi < P.nn, kSiteHeat, gi)) continue;
-                if (P.esc) {
-                    esc_add<R>(P, gi, 4, w[0][i] * w[1][j] * w[2][k] * mT);
-                    esc_mark<R>(P, gx, gy, gz);
-                } else {
-                    atomicAdd(&tw[gi], w[0][i] * w[1][j] * w[2][k] * mT);
-                }
-            }
-        }
-    }
-}
-
+// Heat conduction of a particle whose stencil left the bin tile: the
+// temperature gather over the nodes with m > 1e-18 (sum of w T and of w), as
+// the tile path does.
 template <typename R> struct TSum {
     R ts, ws;
 };
@@ -1059,6 +1023,7 @@ template <typename R, bool EXT> struct StepSmem {
     V4<R> acc[kWarps][kTileSlots];
     V4<R> stage[sizeof(R) == 4 ? kStageGroups : 1][sizeof(R) == 4 ? kNT : 1];
     R nT[EXT ? kWarps : 1][EXT ? kPlane : 1];   // T m (tidx layout), the same way
+    V4<R> far_nv[kWarps][27];   // the node velocities of a particle off the tile
     // node temperatures and their m > 1e-18 mask (0 or 1) as pairs (pidx)
     P2T<R> ttile[EXT ? kPairSlots : 1];
     // the work item's tool poses at the G2P step (x, y, z) and at the P2G step:
@@ -1077,13 +1042,6 @@ template <typename R, bool EXT> struct StepSmem {
 };
 
 template <typename R, bool EXT> constexpr size_t step_smem_bytes() { return sizeof(StepSmem<R, EXT>); }
-
-// What a particle scatters: its offset from its base node after the move (cells),
-// Q = m (v - dx C d) + f_ext dt, R = m dx C and S = -dt V J sigma / dx
-// (row-major), T absolute (heat conduction).
-template <typename R> struct Payload {
-    R d[3], Q[3], Rm[9], S[9], T;
-};
 
 // Coefficients of two momentum channels (a pair in every operand) over the 27
 // stencil nodes (i,j,k) of a particle, relative to its base node:
@@ -1354,8 +1312,10 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                 const V4<R> b0_ld = G2P ? mk4<R>(0, 0, 0, 0) : (kStage ? x4 : ldcs4(&ps.B[0][pi]));
                 uint8_t st = valid ? st_next : (uint8_t)ST_INACTIVE;
                 Payload<R> pay;
-                bool staged = false;
-                int bc[3] = {0, 0, 0};   // base cell of the staged particle
+                bool staged = false, off = false;   // its particle scatters in the tile, off the tile
+                const unsigned moving =
+                    G2P ? __ballot_sync(0xffffffffu, st != ST_INACTIVE && st != ST_FIXED) : 0u;
+                int bc[3] = {0, 0, 0};   // its base cell
                 if (st != ST_INACTIVE) {
                     const uint8_t st_in = st;
                     const bool fixed = (st == ST_FIXED);
@@ -1392,7 +1352,27 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                             }
                             R M[3][3], L[3][3];
                             TSum<R> tsum{R(0), R(0)};
-                            if (__builtin_expect(b[0] >= 0 && b[0] < kBin && b[1] >= 0 && b[1] < kBin && b[2] >= 0 && b[2] < kBin, 1)) {
+                            const bool in_tile = b[0] >= 0 && b[0] < kBin && b[1] >= 0 && b[1] < kBin && b[2] >= 0 &&
+                                                 b[2] < kBin;
+                            // (the lanes here are those of `moving`)
+                            for (unsigned out = __ballot_sync(moving, !in_tile); MPMB_UNLIKELY(out); out &= out - 1u) {
+                                const int e = __ffs((int)out) - 1;
+                                far_nodes<R>(P, gr, g0x + __shfl_sync(moving, b[0], e), g0y + __shfl_sync(moving, b[1], e),
+                                             g0z + __shfl_sync(moving, b[2], e), pose[0], pose[2], Sm.far_nv[wid],
+                                             __popc(moving & ((1u << lane) - 1u)), __popc(moving));
+                                __syncwarp(moving);
+                                if (lane == e) {
+                                    const GatherOut<R> go = far_sum<R>(Sm.far_nv[wid], d[0], d[1], d[2]);
+#pragma unroll
+                                    for (int c = 0; c < 3; ++c) {
+                                        v[c] = go.v[c];
+#pragma unroll
+                                        for (int q = 0; q < 3; ++q) { M[c][q] = go.M[c][q]; L[c][q] = go.L[c][q]; }
+                                    }
+                                }
+                                __syncwarp(moving);
+                            }
+                            if (__builtin_expect(in_tile, 1)) {
                                 gather_tile<R>(Sm.vel, Stencil(b[0], b[1], b[2]), w, dw, v, M, L);
                                 if (EXT && P.heat_on) {
                                     const P2T<R>* tb = Sm.ttile + pidx(b[0], b[1], b[2]);
@@ -1410,14 +1390,6 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                                     tsum.ws = hi2(sum);
                                 }
                             } else {
-                                const GatherOut<R> go = gather_global<R>(P, gr, g0x, g0y, g0z, xi[0], xi[1], xi[2],
-                                                                         pose[0], pose[2]);
-#pragma unroll
-                                for (int c = 0; c < 3; ++c) {
-                                    v[c] = go.v[c];
-#pragma unroll
-                                    for (int q = 0; q < 3; ++q) { M[c][q] = go.M[c][q]; L[c][q] = go.L[c][q]; }
-                                }
                                 ++c_esc;
                                 if (EXT && P.heat_on) tsum = gather_T_global<R>(P, gr, g0x, g0y, g0z, xi[0], xi[1], xi[2]);
                             }
@@ -1715,22 +1687,13 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                             if (__builtin_expect(bb[0] >= 0 && bb[0] < kBin && bb[1] >= 0 && bb[1] < kBin && bb[2] >= 0 &&
                                                      bb[2] < kBin, 1)) {
                                 staged = true;
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) bc[a] = bb[a];
-                                if (EXT) pay.T = P.Tamb + dT;   // absolute (heat conduction)
                             } else {
-                                ScatterIn<R> si;
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) { si.xi[a] = xi[a]; si.Q[a] = Q[a]; }
-#pragma unroll
-                                for (int q = 0; q < 9; ++q) { si.Rm[q] = Rm[q]; si.S[q] = S[q]; }
-                                si.g0[0] = g0x; si.g0[1] = g0y; si.g0[2] = g0z;
-                                scatter_global<R>(P, gw, si, m);
-                                if (EXT && P.heat_on)
-                                    scatter_T_global<R>(P, P.tm[rbuf ^ (G2P ? 1 : 0)], g0x, g0y, g0z, xi[0], xi[1],
-                                                        xi[2], m * (P.Tamb + dT));
+                                off = true;
                                 ++c_esc;
                             }
+#pragma unroll
+                            for (int a = 0; a < 3; ++a) bc[a] = bb[a];
+                            if (EXT) pay.T = P.Tamb + dT;   // absolute (heat conduction)
                         }
                     }
 
@@ -1761,6 +1724,21 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                 fetch_fp(base + kNT);
                 if (P2G) {
                     __syncwarp();
+                    for (unsigned far = __ballot_sync(0xffffffffu, off); MPMB_UNLIKELY(far); far &= far - 1u) {
+                        const int e = __ffs((int)far) - 1;
+                        auto from = [&](auto x) { return __shfl_sync(0xffffffffu, x, e); };
+                        Payload<R> p;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) { p.d[a] = from(pay.d[a]); p.Q[a] = from(pay.Q[a]); }
+#pragma unroll
+                        for (int q = 0; q < 9; ++q) { p.Rm[q] = from(pay.Rm[q]); p.S[q] = from(pay.S[q]); }
+                        p.T = EXT ? from(pay.T) : R(0);
+                        const int buf = rbuf ^ (G2P ? 1 : 0);
+                        far_scatter<R>(P, gw, EXT && P.heat_on ? P.tm[buf] : nullptr, g0x + from(bc[0]), g0y + from(bc[1]),
+                                       g0z + from(bc[2]), p, P.pmass, lane);
+                    }
+                    __syncwarp();
+                    if (!staged) bc[0] = bc[1] = bc[2] = 0;
                     warp_scatter<R, EXT>(Sm, wid, lane, staged, bc[0], bc[1], bc[2], pay, P.pmass, P.heat_on != 0);
                 }
         }
