@@ -457,6 +457,14 @@ __device__ __forceinline__ void esc_add(const Inst<R>& P, int64_t gi, int ch, R 
     const double q = fmin(fmax((double)v * P.esc_scale, -4.0e18), 4.0e18);
     atomicAdd(&P.esc[ch * P.esc_stride + gi], (unsigned long long)__double2ll_rn(q));
 }
+// Heat conduction: T m of the rounded mass, so that a node whose escaped mass
+// rounds to nothing gets no heat either (T m rounded by itself could leave
+// heat without mass there, a node temperature without bound).
+template <typename R> __device__ __forceinline__ void esc_add_T(const Inst<R>& P, int64_t gi, R m, R T) {
+    const double units = rint(fmin(fmax((double)m * P.esc_scale, -4.0e18), 4.0e18));
+    const double q = fmin(fmax(units * (double)T, -4.0e18), 4.0e18);
+    atomicAdd(&P.esc[4 * P.esc_stride + gi], (unsigned long long)__double2ll_rn(q));
+}
 // ... and marks the bin whose 4x4x4 core holds node (gx, gy, gz) for k_node_sum.
 template <typename R> __device__ __forceinline__ void esc_mark(const Inst<R>& P, int gx, int gy, int gz) {
     P.esc_flag[gx / kBin + P.nbx * (gy / kBin + P.nby * (gz / kBin))] = 1;
@@ -495,7 +503,7 @@ __device__ __noinline__ void far_scatter(const Inst<R>& P, V4<R>* __restrict__ g
         esc_add<R>(P, gi, 1, p[0]);
         esc_add<R>(P, gi, 2, p[1]);
         esc_add<R>(P, gi, 3, p[2]);
-        if (tw) esc_add<R>(P, gi, 4, ww * (m * in.T));
+        if (tw) esc_add_T<R>(P, gi, ww * m, in.T);
         esc_mark<R>(P, gx, gy, gz);
     } else {
         vec_atomic_add<R>(&grid[gi], ww * m, p[0], p[1], p[2]);
