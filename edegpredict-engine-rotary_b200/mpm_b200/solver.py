@@ -188,8 +188,7 @@ class Solver:
         """Launch shape; deterministic=True (the default) gives the same
         results bit for bit on every run and launch shape, False sums node
         tiles with float atomics (mpm_launch_config.deterministic);
-        pass_size: FP32 particles per pass of the step kernel (128, 256, 512;
-        0: the default)."""
+        pass_size: 128, 256 or 512 (0: 128), accepted and without effect."""
         c = A.MpmLaunchConfig(int(ctas_per_sm), int(sort_every), 1 if use_graph else 0, 1 if deterministic else 0,
                               int(pass_size))
         self._check(self._lib.mpm_set_launch_config(self.h, C.byref(c)))
