@@ -387,10 +387,11 @@ __device__ __forceinline__ void gather_tile(const V4<R>* vel, const Stencil& sl,
 // and updated straight from the grid (rare; the re-bin brings it back).  The
 // lanes of the warp that are here update a node each (rank of n lanes; the
 // velocity and whether the node lies in the domain go to nv), then the
-// particle's lane sums them.  One lane updating its 27 nodes, tool distance in
-// FP64 and all, took about 20 us: as long as a bin, and the particles that
-// leave their bins are those at the tool, so a launch of 0.5 M particles
-// waited 35 us for its last bins.
+// particle's lane sums them.  With one lane updating all 27 nodes, tool
+// distance in FP64 and all, a launch of 0.5 M particles took 108 us with a
+// tool and 73 us without one: the particles that leave their bins are those at
+// the tool, and the launch waits for the bins that hold them.  Shared by the
+// lanes it takes 77 us with the tool.
 template <typename R>
 __device__ __noinline__ void far_nodes(const Inst<R>& P, const V4<R>* __restrict__ grid, int gx0, int gy0, int gz0,
                                        double pr0, double pr2, V4<R>* nv, int rank, int n) {
