@@ -1280,10 +1280,13 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
                 // has returned, into shared memory that the SM's next CTA may
                 // own.  The error word is never cleared: every later status or
                 // metrics call on the handle returns MPM_TIMEOUT, and the
-                // caller is expected to stop using it.
+                // caller is expected to stop using it.  The CTA leaves by the
+                // end of the kernel, as every CTA has to: one that did not
+                // count itself out would leave the tickets of this launch to
+                // the next, whose CTAs would then skip bins or take one twice.
                 if (kStage) async_wait<0>();
                 if (tid == 0) atomicOr(err, ERR_TIMEOUT);
-                return;
+                break;
             }
             for (int nidx = tid; nidx < kTileNodes; nidx += kNT) {
                 const int lx = nidx % kTile, ly = (nidx / kTile) % kTile, lz = nidx / (kTile * kTile);
@@ -1788,7 +1791,8 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
         }
         __syncthreads();
     }
-    // the launch's last CTA leaves the counter at zero for the next launch
+    // every CTA counts itself out, and the launch's last one leaves the counter
+    // at zero for the next launch
     if (tid == 0 && atomicAdd(&ticket[1], 1u) == gridDim.x - 1) {
         ticket[0] = 0u;
         ticket[1] = 0u;
