@@ -26,6 +26,7 @@
 
 #include "mpm_device.cuh"
 #include "mpm_internal.h"
+#include "mpm_per_device.h"
 
 namespace mpmb {
 
@@ -1822,28 +1823,22 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
     else if (errf < 0) atomicOr(err, ERR_NEWTON);
 }
 
-// Sets the variant's shared-memory size once and returns how many of its
-// CTAs fit on one SM.  The work loop hands every CTA of the grid the same
-// share of the work items, so a grid with more CTAs than fit would run its
-// last CTAs as a second wave: launches clamp the grid to this.
-template <typename R, bool G2P, bool P2G, bool EXT> static int set_smem_attr() {
-    static bool attr = false;
-    static int fit = 0;
-    if (!attr) {
+// Sets the variant's shared-memory size on the current device `dev` and returns
+// how many of its CTAs fit on one SM (once per device).  A CTA takes its first
+// work item by its own index, so the CTAs of a grid larger than what fits
+// would hold theirs back until another CTA ends: launches clamp the grid to this.
+template <typename R, bool G2P, bool P2G, bool EXT> static int ctas_that_fit(int dev) {
+    static PerDevice fit;
+    const int n = fit.get(dev, [] {
+        int k = 0;
         cudaFuncSetAttribute(k_step<R, G2P, P2G, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)step_smem_bytes<R, EXT>());
-        attr = true;
-    }
-    if (!fit) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_step<R, G2P, P2G, EXT>, kNT,
-                                                          step_smem_bytes<R, EXT>()) == cudaSuccess &&
-            n >= 1)
-            fit = n;
-        else
-            return 8;   // not known (the query failed): no clamp this time, asked again next launch
-    }
-    return fit;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_step<R, G2P, P2G, EXT>, kNT,
+                                                             step_smem_bytes<R, EXT>()) == cudaSuccess
+                   ? k
+                   : 0;
+    });
+    return n > 0 ? n : 8;   // not known (the query failed): no clamp this time
 }
 
 // Deterministic mode, the grid of one P2G: one thread per node of a bin's
@@ -1933,9 +1928,9 @@ void launch_node_sum(const Inst<R>* insts, const int32_t* bin_inst, const int32_
 // at most as many as fit, at most one per work item.
 template <typename R, bool G2P, bool P2G, bool EXT>
 static void launch_variant(const Inst<R>* insts, const Work* work, const int* n_work, const PState<R>& ps,
-                           const StepArgs& a, int rbuf, int sms, int cps, int max_work, int* err,
+                           const StepArgs& a, int rbuf, int dev, int sms, int cps, int max_work, int* err,
                            unsigned long long* counters, unsigned int* ticket, cudaStream_t st) {
-    const int fit = set_smem_attr<R, G2P, P2G, EXT>();
+    const int fit = ctas_that_fit<R, G2P, P2G, EXT>(dev);
     const int grid = std::max(1, std::min(sms * std::min(cps, fit), max_work));
     k_step<R, G2P, P2G, EXT><<<grid, kNT, step_smem_bytes<R, EXT>(), st>>>(insts, work, n_work, ps, a, rbuf, err,
                                                                           counters, ticket);
@@ -1947,18 +1942,19 @@ void launch_step(const Inst<R>* insts, const Work* work, const int* n_work, int 
                  unsigned long long* counters, unsigned int* ticket, cudaStream_t st) {
     (void)threads;
     Range nvtx_range(g2p && p2g ? "mpm.launch.g2p_p2g" : (g2p ? "mpm.launch.g2p" : "mpm.launch.p2g"));
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static PerDevice sm_count;
+    int sms = sm_count.get(dev, [dev] {
+        int n = 0;
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 0;
+    });
+    if (sms <= 0) sms = 148;
     if (max_work <= 0) return;
     const int cps = ctas_per_sm > 0 ? ctas_per_sm : 4;
     auto go = [&](auto g, auto p, auto e) {
         launch_variant<R, decltype(g)::value, decltype(p)::value, decltype(e)::value>(
-            insts, work, n_work, ps, a, rbuf, sms, cps, max_work, err, counters, ticket, st);
+            insts, work, n_work, ps, a, rbuf, dev, sms, cps, max_work, err, counters, ticket, st);
     };
     using T = std::true_type;
     using F = std::false_type;
