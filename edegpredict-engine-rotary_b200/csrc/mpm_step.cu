@@ -1098,8 +1098,9 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
     unsigned todo = __ballot_sync(0xffffffffu, staged);
     if (todo == 0u) return;
     const Stencil sl(bx, by, bz);
-    V4<R>* __restrict__ tile = Sm.acc[wid];
-    R* __restrict__ nt = Sm.nT[EXT ? wid : 0] + (EXT ? tidx(bx, by, bz) : 0);
+    // (not __restrict__: the other lanes write the same nodes between the phases)
+    V4<R>* tile = Sm.acc[wid];
+    R* nt = Sm.nT[EXT ? wid : 0] + (EXT ? tidx(bx, by, bz) : 0);
     const R mT = EXT ? pm * p.T : R(0);
     P2 w[3][3];
     R w1[3][3], dw[3][3];

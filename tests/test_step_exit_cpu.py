@@ -39,3 +39,12 @@ def test_every_cta_counts_itself_out():
     assert not re.search(r"\b(exit|__trap)\b", body)
     loop, tail = body.index("blockIdx.x; wi < nw"), body.index("atomicAdd(&ticket[1], 1u)")
     assert loop < tail and body.count("ticket[1], 1u") == 1
+
+
+def test_the_scatter_does_not_promise_its_tile_to_itself():
+    """The lanes of a warp add to the same nodes in turns, ordered by
+    __syncwarp alone: a __restrict__ on the tile would let a compiler move a
+    load over another lane's store."""
+    src = re.sub(r"//[^\n]*", "", STEP.read_text())
+    body = block(src, src.index("{", src.index("void warp_scatter(")))
+    assert "Sm.acc[wid]" in body and "__restrict__" not in body
