@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "mpm_engine.h"
+#include "mpm_flow_bound.h"
 #include "mpm_checkpoint.h"
 
 namespace mpmb {
@@ -702,8 +703,9 @@ class Engine final : public EngineBase {
             d.ylo = (p.jc_A > 0.0 && p.jc_B >= 0.0 && p.jc_C >= 0.0 && rt_lo > 0.0)
                         ? (R)(p.jc_A * rt_lo * (1.0 - 1e-4))
                         : R(0);
-            // (the same margin again for the rounding of 1 - Ts^m and of the bound)
-            d.ymin = p.jc_m > 0.0 ? (R)((double)d.ylo * std::min(p.jc_m, 1.0) * (1.0 - 1e-4)) : R(0);
+            const FlowBound<R> b = flow_bound<R>(d.ylo, p.jc_m);
+            d.ymin = b.scale;
+            d.yslack = b.slack;
         }
         d.dTmax = (R)(p.Tm - p.Tamb);
         d.heat = (R)(p.beta / std::max(p.rho_phys * p.cp, 1e-12));

@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "mpm_device.cuh"
+#include "mpm_flow_bound.h"
 #include "mpm_internal.h"
 #include "mpm_per_device.h"
 
@@ -792,10 +793,9 @@ __device__ __forceinline__ JCOut jc_update(const Inst<R>& P, const R H[9], R Hp[
     // a particle with q below the smallest flow stress the step can have
     // (ylo tt, heated or not: ylo bounds (A + B eps^n)(1 + C ln es) from
     // below, tt = 1 - Ts^m the thermal factor) cannot yield: the flow stress
-    // itself is not needed.  Ts^m lies below its chord (m >= 1) or its tangent
-    // at Ts = 1 (m < 1), so tt >= min(m, 1) (1 - Ts): ymin holds ylo min(m, 1)
-    // and most particles, heated or not, take no power.
-    if (__builtin_expect(q < P.ymin * (R(1) - Ts), 1)) return o;
+    // itself is not needed.  flow_bound_at lies below ylo tt, so most
+    // particles, heated or not, take no power either.
+    if (__builtin_expect(q < flow_bound_at(P.ymin, P.yslack, Ts), 1)) return o;
     // (pow(0, y) is +0 for y > 0)
     const R tt = R(1) - ((Ts > R(0) || !(P.m > R(0))) ? pow(Ts, P.m) : R(0));
     if (q < P.ylo * tt) return o;
