@@ -13,8 +13,9 @@
 #include <vector>
 
 #include "mpm_engine.h"
-#include "mpm_flow_bound.h"
 #include "mpm_checkpoint.h"
+#include "mpm_flow_bound.h"
+#include "mpm_pinned.h"
 
 namespace mpmb {
 
@@ -37,6 +38,37 @@ PFN_encodeTiled_t encode_fn() {
     return fn;
 }
 
+struct PinnedOps {
+    bool context(uint64_t* id) {
+        typedef CUresult (*PFN_ctxGetId_t)(CUcontext, unsigned long long*);
+        static const PFN_ctxGetId_t fn = [] {
+            void* p = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            return cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                           q == cudaDriverEntryPointSuccess
+                       ? (PFN_ctxGetId_t)p
+                       : nullptr;
+        }();
+        unsigned long long v = 0;
+        if (!fn || fn(nullptr, &v) != CUDA_SUCCESS) return false;
+        *id = v;
+        return true;
+    }
+    void* alloc(size_t bytes) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    void release(void* p) { cudaFreeHost(p); }
+};
+// (never destroyed: handles may close while the process's statics go)
+PinnedSlots<PinnedOps>& pinned_slots() {
+    static PinnedSlots<PinnedOps>* const slots = new PinnedSlots<PinnedOps>();
+    return *slots;
+}
+static_assert(sizeof(ReadBack) <= PinnedSlots<PinnedOps>::kSlotBytes, "a slot holds a read-back");
+
 inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 #define CK(call)                                                                                     \
@@ -55,6 +87,9 @@ inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
     } while (0)
 
 }  // namespace
+
+void* pinned_take() { return pinned_slots().take(); }
+void pinned_give(void* slot) { pinned_slots().give(slot); }
 
 mpm_status check_params(const mpm_params* p, std::string* err) {
     auto bad = [&](const char* m) {
@@ -127,7 +162,7 @@ class Engine final : public EngineBase {
     unsigned int* d_ticket = nullptr;   // work-item tickets of the step kernel, zero between launches
     static constexpr size_t kCtrBytes = kCounters * sizeof(unsigned long long);
     double* d_stat_part = nullptr;
-    ReadBack* h_rb = nullptr;      // pinned
+    ReadBack* h_rb = nullptr;      // a pinned slot
     int stat_blocks = 0;
     void* d_stage = nullptr;
     size_t stage_bytes = 0;
@@ -206,7 +241,7 @@ class Engine final : public EngineBase {
                         d_map, d_perm, d_part, d_esc, d_esc_flag, d_pext, d_flags, d_ticket};
         for (void* p : ptrs)
             if (p) cudaFree(p);
-        if (h_rb) cudaFreeHost(h_rb);
+        if (h_rb) pinned_give(h_rb);   // (the stream has run dry above)
         for (auto& x : I)
             if (x.d_samples) cudaFree(x.d_samples);
         for (auto e : ev_pool) cudaEventDestroy(e);
@@ -248,7 +283,11 @@ class Engine final : public EngineBase {
         CK(cudaMemsetAsync(d_ticket, 0, 2 * sizeof(unsigned int), st));
         stat_blocks = 148 * 8;   // 8 CTAs per SM of the metrics reduction (more loads in flight)
         CK(cudaMalloc(&d_stat_part, sizeof(double) * kStatSlots * stat_blocks));
-        CK(cudaHostAlloc(&h_rb, sizeof(ReadBack), cudaHostAllocDefault));
+        h_rb = static_cast<ReadBack*>(pinned_take());
+        if (!h_rb) {
+            err = "no pinned host memory";
+            return MPM_OOM;
+        }
         return relayout(std::move(nI), std::vector<int>(n, -1));
     }
 
