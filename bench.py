@@ -1014,7 +1014,7 @@ def main():
     ap.add_argument("--sort-every", type=int, default=0,
                     help="plain configs: steps between re-bins (0: the default, 16)")
     ap.add_argument("--pass-size", type=int, default=0, choices=[0, 128, 256, 512],
-                    help="plain configs: FP32 particles per pass of the step kernel (0: the default)")
+                    help="plain configs: the launch config's pass_size (accepted, without effect)")
     ap.add_argument("--atomic", action="store_true",
                     help="plain configs and precision_study: add node tiles with FP32 atomics instead of the "
                          "default deterministic node sums")

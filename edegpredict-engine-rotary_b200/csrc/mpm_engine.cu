@@ -177,8 +177,8 @@ class Engine final : public EngineBase {
     int64_t n_sorts = 0;
     int64_t launch_base = 0;
     int sort_every = 16, threads = 128, ctas_per_sm = 4, prec_ = MPM_PREC_F32;
-    static constexpr int kDefaultPassChunk = 1;
-    int pass_chunk = kDefaultPassChunk;   // the launch config's pass_size / 128 (kept, no effect)
+    static constexpr int kDefaultPassSize = 128;
+    int pass_size = kDefaultPassSize;   // of the launch config: kept, no effect
     bool use_graph = false;
     int rbuf = 0;
     // deterministic mode (mpm_launch_config.deterministic): every work item's
@@ -1581,7 +1581,7 @@ class Engine final : public EngineBase {
         c->sort_every = sort_every;
         c->use_graph = use_graph ? 1 : 0;
         c->deterministic = det ? 1 : 0;
-        c->pass_size = pass_chunk * 128;
+        c->pass_size = pass_size;
         return MPM_OK;
     }
 
@@ -1593,11 +1593,9 @@ class Engine final : public EngineBase {
                   "0, 128, 256 or 512";
             return MPM_INVALID_ARG;
         }
-        const int chunk = c->pass_size ? c->pass_size / 128 : kDefaultPassChunk;
-        if (c->ctas_per_sm != ctas_per_sm || c->sort_every != sort_every || (c->deterministic != 0) != det ||
-            chunk != pass_chunk)
+        if (c->ctas_per_sm != ctas_per_sm || c->sort_every != sort_every || (c->deterministic != 0) != det)
             drop_graphs();
-        pass_chunk = chunk;
+        pass_size = c->pass_size ? c->pass_size : kDefaultPassSize;
         det = c->deterministic != 0;
         ctas_per_sm = c->ctas_per_sm;
         sort_every = c->sort_every;
@@ -1606,12 +1604,10 @@ class Engine final : public EngineBase {
         return MPM_OK;
     }
 
-    // Times the candidates over real steps and keeps the fastest: the pass
-    // size first (16 steps each at the current CTAs and cadence), then, at the
-    // fastest pass size, CTAs per SM x re-bin cadence over one re-bin period
-    // each.  The trial steps advance the simulation like any other steps.
+    // Times the candidates, CTAs per SM x re-bin cadence, over one re-bin period
+    // each of real steps and keeps the fastest.  The trial steps advance the
+    // simulation like any other steps.
     mpm_status autotune(const double* dts, mpm_launch_config* best) override {
-        const int cand_pass[3] = {128, 256, 512};
         const int cand_ctas[3] = {2, 3, 4};
         const int cand_sort[3] = {8, 16, 32};
         mpm_launch_config cur_cfg{};
@@ -1641,22 +1637,9 @@ class Engine final : public EngineBase {
             return MPM_OK;
         };
         mpm_status s = MPM_OK;
-        for (int a = 0; a < 3 && s == MPM_OK; ++a) {
-            mpm_launch_config c = cur_cfg;
-            c.pass_size = cand_pass[a];
-            double per = 0.0;
-            if ((s = trial(c, 16, &per)) != MPM_OK) break;
-            if (per < win_ms) {
-                win_ms = per;
-                win = c;
-            }
-        }
-        const int pass = win.pass_size;
-        win_ms = 1e300;
         for (int a = 0; a < 3 && s == MPM_OK; ++a)
             for (int b = 0; b < 3 && s == MPM_OK; ++b) {
                 mpm_launch_config c = cur_cfg;
-                c.pass_size = pass;
                 c.ctas_per_sm = cand_ctas[a];
                 c.sort_every = cand_sort[b];
                 double per = 0.0;

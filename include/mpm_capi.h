@@ -521,11 +521,9 @@ typedef struct mpm_launch_config {
 mpm_status mpm_get_launch_config(const mpm_handle *h, mpm_launch_config *out);
 mpm_status mpm_set_launch_config(mpm_handle *h, const mpm_launch_config *cfg);
 /* Picks the launch shape by timing real steps (dt[i] per instance, counted
- * like any other steps): first the pass size (128, 256, 512 FP32 particles,
- * 16 steps each at the current CTAs and cadence), then, at the fastest pass
- * size, every CTAs per SM in {2,3,4} x re-bin every {8,16,32} steps over one
- * re-bin period each (216 steps in all).  Keeps the fastest; *chosen (may be
- * NULL) receives it. */
+ * like any other steps): every CTAs per SM in {2,3,4} x re-bin every {8,16,32}
+ * steps over one re-bin period each (168 steps in all).  Keeps the fastest;
+ * *chosen (may be NULL) receives it. */
 mpm_status mpm_autotune(mpm_handle *h, const double *dt, mpm_launch_config *chosen);
 
 /*

@@ -134,8 +134,8 @@ def test_graph_replay_and_autotune_keep_results():
         cfg = bt.autotune(dts)
         assert cfg["ctas_per_sm"] in (2, 3, 4) and cfg["sort_every"] in (8, 16, 32)
         assert cfg["pass_size"] in (128, 256, 512)
-        # 16 steps per pass size, then one re-bin period per CTAs x cadence
-        assert bt.counts_i(0)[1] == 12 + 3 * 16 + 3 * (8 + 16 + 32)
+        # one re-bin period per CTAs x cadence
+        assert bt.counts_i(0)[1] == 12 + 3 * (8 + 16 + 32)
     finally:
         bt.close()
     for i, c in enumerate(cases):
