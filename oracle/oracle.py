@@ -338,13 +338,17 @@ class Oracle:
         return np.array(out[:], dtype=np.float32)
 
 
+class ReferenceMissing(RuntimeError):
+    """The reference's own kernels are not built here."""
+
+
 class RefKern:
     """The reference's own CUDA kernels (needs a GPU)."""
 
     def __init__(self):
         if not REF_LIB.exists():
-            raise RuntimeError(f"{REF_LIB} is missing: build it with `make -C oracle ref` where the reference "
-                               "sources are present")
+            raise ReferenceMissing(f"{REF_LIB} is missing: build it with `make -C oracle ref` where the reference "
+                                   "sources are present")
         L = C.CDLL(str(REF_LIB))
         L.ref_last_error.restype = C.c_char_p
         L.ref_device_count.restype = _i32
