@@ -1433,7 +1433,7 @@ class Engine final : public EngineBase {
                 raster_all(k);
                 diffuse(w);
                 StepArgs c{k, 1, 0, 0, k, xk};
-                    prof_begin();
+                prof_begin();
                 launch_step<R>(d_inst, d_work, d_nwork, max_work, ps[cur], c, w, true, false, threads, cps, d_err,
                                d_ctr, d_ticket, st);
                 prof_end();

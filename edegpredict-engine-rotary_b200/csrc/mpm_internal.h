@@ -96,7 +96,7 @@ void launch_bin_count(const Inst<R>* insts, int n_inst, const PState<R>& ps, con
                       int64_t np, int kpt, int sort_every, bool keep_all, cudaStream_t st);
 
 // The re-bin's move: every particle to its slot in the new layout, each
-// cell's particles in the order of their old slots (bin_key: the first key
+// cell's particles in the order of their upload positions (bin_key: the first key
 // of each of the nbins_total bins of the bin table).  mid_call: inside a fused
 // step call, where B of ACTIVE particles is dead and stays behind.
 template <typename R>

@@ -540,6 +540,7 @@ __device__ __noinline__ TSum<R> gather_T_global(const Inst<R>& P, const V4<R>* _
                 const int gz = gb[2] + k;
                 if (gz < 0 || gz >= P.nz) continue;
                 const int64_t q = gx + (int64_t)P.nx * (gy + (int64_t)P.ny * gz);
+                if (!MPMB_CHECK(q >= 0 && q < P.nn, kSiteHeat, q)) continue;
                 const R ww = w[0][i] * w[1][j] * w[2][k];
                 if (!(ww > R(0)) || !(grid[q].x > R(1e-18))) continue;
                 o.ts += P.tn[q] * ww;
@@ -1121,35 +1122,35 @@ __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int 
             mine = (__ffs((int)__match_any_sync(todo, bx + kBin * (by + kBin * bz))) - 1) == lane;
         todo &= ~__ballot_sync(0xffffffffu, mine);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        P2 PA[3], PB[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            PA[k] = fma2(w[0][i], A.Az[k], mul2(A.Bx[i], w[2][k]));
-            PB[k] = fma2(w[0][i], B.Az[k], mul2(B.Bx[i], w[2][k]));
-        }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const P2 QA = mul2(w[0][i], A.Cy[j]), QB = mul2(w[0][i], B.Cy[j]);
-            V4<R>* n = tile + sl.at(i, j) + kRow * j;
-            const R mxy = EXT ? mT * w1[0][i] * w1[1][j] : R(0);
-            auto added = [&](const V4<R>& o, int k) {
-                const P2 a = fma2(w[1][j], PA[k], fma2(QA, w[2][k], mk2(o.x, o.y)));
-                const P2 b = fma2(w[1][j], PB[k], fma2(QB, w[2][k], mk2(o.z, o.w)));
-                return mk4<R>(lo2(a), hi2(a), lo2(b), hi2(b));
-            };
+        for (int i = 0; i < 3; ++i) {
+            P2 PA[3], PB[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                __syncwarp();
-                if (mine) {
-                    n[kLayer * k] = added(n[kLayer * k], k);
-                    // heat conduction: the T m channel, w m T
-                    if (EXT && heat) nt[i + kSY * j + kSZ * k] = fma(mxy, w1[2][k], nt[i + kSY * j + kSZ * k]);
+                PA[k] = fma2(w[0][i], A.Az[k], mul2(A.Bx[i], w[2][k]));
+                PB[k] = fma2(w[0][i], B.Az[k], mul2(B.Bx[i], w[2][k]));
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const P2 QA = mul2(w[0][i], A.Cy[j]), QB = mul2(w[0][i], B.Cy[j]);
+                V4<R>* n = tile + sl.at(i, j) + kRow * j;
+                const R mxy = EXT ? mT * w1[0][i] * w1[1][j] : R(0);
+                auto added = [&](const V4<R>& o, int k) {
+                    const P2 a = fma2(w[1][j], PA[k], fma2(QA, w[2][k], mk2(o.x, o.y)));
+                    const P2 b = fma2(w[1][j], PB[k], fma2(QB, w[2][k], mk2(o.z, o.w)));
+                    return mk4<R>(lo2(a), hi2(a), lo2(b), hi2(b));
+                };
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    __syncwarp();
+                    if (mine) {
+                        n[kLayer * k] = added(n[kLayer * k], k);
+                        // heat conduction: the T m channel, w m T
+                        if (EXT && heat) nt[i + kSY * j + kSZ * k] = fma(mxy, w1[2][k], nt[i + kSY * j + kSZ * k]);
+                    }
                 }
             }
         }
-    }
-    __syncwarp();
+        __syncwarp();
     } while (todo);
 }
 
@@ -1313,448 +1314,448 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
         // The warps run their rounds of 32 particles independently: no CTA
         // barrier until the end of the bin.
         for (int base = 0; base + (wid << 5) < wk.count; base += kNT) {
-                const int64_t pi = slot_of(base);
-                const bool valid = base + tid < wk.count &&
-                                   MPMB_CHECK(pi >= P.pbase && pi < P.pbase + P.pcap, kSiteParticle, pi);
-                if (kStage) async_wait<P2G ? 1 : 0>();   // this round's head (its F_p group may be pending)
-                const V4<R> a0 = kStage ? Sm.stage[0][tid] : ldcs4(&ps.A[0][pi]),
-                            a1 = kStage ? Sm.stage[kStage ? 1 : 0][tid] : ldcs4(&ps.A[1][pi]),
-                            a2 = kStage ? Sm.stage[kStage ? 2 : 0][tid] : ldcs4(&ps.A[2][pi]),
-                            a3 = kStage ? Sm.stage[kStage ? 3 : 0][tid] : ldcs4(&ps.A[3][pi]);
-                const V4<R> x4 = kStage ? Sm.stage[kStage ? 4 : 0][tid] : mk4<R>(0, 0, 0, 0);
-                const V4<R> xl = G2P ? x4 : mk4<R>(0, 0, 0, 0);
-                const V4<R> b0_ld = G2P ? mk4<R>(0, 0, 0, 0) : (kStage ? x4 : ldcs4(&ps.B[0][pi]));
-                uint8_t st = valid ? st_next : (uint8_t)ST_INACTIVE;
-                Payload<R> pay;
-                bool staged = false, off = false;   // its particle scatters in the tile, off the tile
-                const unsigned moving =
-                    G2P ? __ballot_sync(0xffffffffu, st != ST_INACTIVE && st != ST_FIXED) : 0u;
-                int bc[3] = {0, 0, 0};   // its base cell
-                if (st != ST_INACTIVE) {
-                    const uint8_t st_in = st;
-                    const bool fixed = (st == ST_FIXED);
-                    R xi[3] = {a0.x, a0.y, a0.z};
-                    R eps = a0.w;
-                    R H[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
-                    R Hp8 = a3.y, dT = a3.z, Dm = a3.w;
-                    // low parts of the position (FP32 state); the move is an exact two-sum
-                    R lo[3] = {R(0), R(0), R(0)};
-                    const bool has_lo = G2P && !fixed && ps.X != nullptr;
-                    if (has_lo) { lo[0] = xl.x; lo[1] = xl.y; lo[2] = xl.z; }
-                    R v[3] = {0, 0, 0}, Cm[9], edot = R(0);
-                    bool have_C = false, dirtyA = false, wrote_C = false;
+            const int64_t pi = slot_of(base);
+            const bool valid = base + tid < wk.count &&
+                               MPMB_CHECK(pi >= P.pbase && pi < P.pbase + P.pcap, kSiteParticle, pi);
+            if (kStage) async_wait<P2G ? 1 : 0>();   // this round's head (its F_p group may be pending)
+            const V4<R> a0 = kStage ? Sm.stage[0][tid] : ldcs4(&ps.A[0][pi]),
+                        a1 = kStage ? Sm.stage[kStage ? 1 : 0][tid] : ldcs4(&ps.A[1][pi]),
+                        a2 = kStage ? Sm.stage[kStage ? 2 : 0][tid] : ldcs4(&ps.A[2][pi]),
+                        a3 = kStage ? Sm.stage[kStage ? 3 : 0][tid] : ldcs4(&ps.A[3][pi]);
+            const V4<R> x4 = kStage ? Sm.stage[kStage ? 4 : 0][tid] : mk4<R>(0, 0, 0, 0);
+            const V4<R> xl = G2P ? x4 : mk4<R>(0, 0, 0, 0);
+            const V4<R> b0_ld = G2P ? mk4<R>(0, 0, 0, 0) : (kStage ? x4 : ldcs4(&ps.B[0][pi]));
+            uint8_t st = valid ? st_next : (uint8_t)ST_INACTIVE;
+            Payload<R> pay;
+            bool staged = false, off = false;   // its particle scatters in the tile, off the tile
+            const unsigned moving =
+                G2P ? __ballot_sync(0xffffffffu, st != ST_INACTIVE && st != ST_FIXED) : 0u;
+            int bc[3] = {0, 0, 0};   // its base cell
+            if (st != ST_INACTIVE) {
+                const uint8_t st_in = st;
+                const bool fixed = (st == ST_FIXED);
+                R xi[3] = {a0.x, a0.y, a0.z};
+                R eps = a0.w;
+                R H[9] = {a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z, a2.w, a3.x};
+                R Hp8 = a3.y, dT = a3.z, Dm = a3.w;
+                // low parts of the position (FP32 state); the move is an exact two-sum
+                R lo[3] = {R(0), R(0), R(0)};
+                const bool has_lo = G2P && !fixed && ps.X != nullptr;
+                if (has_lo) { lo[0] = xl.x; lo[1] = xl.y; lo[2] = xl.z; }
+                R v[3] = {0, 0, 0}, Cm[9], edot = R(0);
+                bool have_C = false, dirtyA = false, wrote_C = false;
 
-                    if (G2P) {
-                        if (!fixed) {
-                            bool far = false;
-                            if (MPMB_UNLIKELY(P.lod && st == ST_ACTIVE)) {
-                                const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - pose[0];
-                                const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - pose[1];
-                                const double wz =
-                                    P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - (pose[2] + P.tool_tip_dz);
-                                far = sqrt(wx * wx + wy * wy + wz * wz) > P.lod_r2;
+                if (G2P) {
+                    if (!fixed) {
+                        bool far = false;
+                        if (MPMB_UNLIKELY(P.lod && st == ST_ACTIVE)) {
+                            const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - pose[0];
+                            const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - pose[1];
+                            const double wz =
+                                P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - (pose[2] + P.tool_tip_dz);
+                            far = sqrt(wx * wx + wy * wy + wz * wz) > P.lod_r2;
+                        }
+                        R w[3][3], dw[3][3];
+                        int b[3];
+                        R d[3];
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            const R fb = floor(xi[a] - R(0.5));
+                            d[a] = xi[a] - fb;
+                            b[a] = (int)fb;
+                            bspline_at(d[a], w[a], dw[a]);
+                        }
+                        R M[3][3], L[3][3];
+                        TSum<R> tsum{R(0), R(0)};
+                        const bool in_tile = b[0] >= 0 && b[0] < kBin && b[1] >= 0 && b[1] < kBin && b[2] >= 0 &&
+                                             b[2] < kBin;
+                        // (the lanes here are those of `moving`)
+                        for (unsigned out = __ballot_sync(moving, !in_tile); MPMB_UNLIKELY(out); out &= out - 1u) {
+                            const int e = __ffs((int)out) - 1;
+                            far_nodes<R>(P, gr, g0x + __shfl_sync(moving, b[0], e), g0y + __shfl_sync(moving, b[1], e),
+                                         g0z + __shfl_sync(moving, b[2], e), pose[0], pose[2], Sm.far_nv[wid],
+                                         __popc(moving & ((1u << lane) - 1u)), __popc(moving));
+                            __syncwarp(moving);
+                            if (lane == e) {
+                                const GatherOut<R> go = far_sum<R>(Sm.far_nv[wid], d[0], d[1], d[2]);
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) {
+                                    v[c] = go.v[c];
+#pragma unroll
+                                    for (int q = 0; q < 3; ++q) { M[c][q] = go.M[c][q]; L[c][q] = go.L[c][q]; }
+                                }
                             }
-                            R w[3][3], dw[3][3];
-                            int b[3];
-                            R d[3];
+                            __syncwarp(moving);
+                        }
+                        if (__builtin_expect(in_tile, 1)) {
+                            gather_tile<R>(Sm.vel, Stencil(b[0], b[1], b[2]), w, dw, v, M, L);
+                            if (EXT && P.heat_on) {
+                                const P2T<R>* tb = Sm.ttile + pidx(b[0], b[1], b[2]);
+                                P2T<R> sum = dup2(R(0));   // (sum w T, sum w) over the counted nodes
 #pragma unroll
-                            for (int a = 0; a < 3; ++a) {
-                                const R fb = floor(xi[a] - R(0.5));
-                                d[a] = xi[a] - fb;
-                                b[a] = (int)fb;
-                                bspline_at(d[a], w[a], dw[a]);
-                            }
-                            R M[3][3], L[3][3];
-                            TSum<R> tsum{R(0), R(0)};
-                            const bool in_tile = b[0] >= 0 && b[0] < kBin && b[1] >= 0 && b[1] < kBin && b[2] >= 0 &&
-                                                 b[2] < kBin;
-                            // (the lanes here are those of `moving`)
-                            for (unsigned out = __ballot_sync(moving, !in_tile); MPMB_UNLIKELY(out); out &= out - 1u) {
-                                const int e = __ffs((int)out) - 1;
-                                far_nodes<R>(P, gr, g0x + __shfl_sync(moving, b[0], e), g0y + __shfl_sync(moving, b[1], e),
-                                             g0z + __shfl_sync(moving, b[2], e), pose[0], pose[2], Sm.far_nv[wid],
-                                             __popc(moving & ((1u << lane) - 1u)), __popc(moving));
-                                __syncwarp(moving);
-                                if (lane == e) {
-                                    const GatherOut<R> go = far_sum<R>(Sm.far_nv[wid], d[0], d[1], d[2]);
+                                for (int k = 0; k < 3; ++k)
 #pragma unroll
-                                    for (int c = 0; c < 3; ++c) {
-                                        v[c] = go.v[c];
+                                    for (int j = 0; j < 3; ++j) {
+                                        const R wjk = w[1][j] * w[2][k];
 #pragma unroll
-                                        for (int q = 0; q < 3; ++q) { M[c][q] = go.M[c][q]; L[c][q] = go.L[c][q]; }
+                                        for (int i = 0; i < 3; ++i)
+                                            sum = fma2(dup2(w[0][i] * wjk), tb[EXT ? pidx(i, j, k) : 0], sum);
                                     }
-                                }
-                                __syncwarp(moving);
+                                tsum.ts = lo2(sum);
+                                tsum.ws = hi2(sum);
                             }
-                            if (__builtin_expect(in_tile, 1)) {
-                                gather_tile<R>(Sm.vel, Stencil(b[0], b[1], b[2]), w, dw, v, M, L);
-                                if (EXT && P.heat_on) {
-                                    const P2T<R>* tb = Sm.ttile + pidx(b[0], b[1], b[2]);
-                                    P2T<R> sum = dup2(R(0));   // (sum w T, sum w) over the counted nodes
+                        } else {
+                            ++c_esc;
+                            if (EXT && P.heat_on) tsum = gather_T_global<R>(P, gr, g0x, g0y, g0z, xi[0], xi[1], xi[2]);
+                        }
+                        if (EXT && P.heat_on && tsum.ws > R(1e-8)) {
+                            // heat conduction: the temperature gather of mpmG2PKernel
+                            // (src/MPMWorkpieceSolver.cu:282-306), clamped to [Tamb, Tm]
+                            dT = fmin(fmax(tsum.ts / tsum.ws, P.Tamb), P.Tamb + P.dTmax) - P.Tamb;
+                        }
 #pragma unroll
-                                    for (int k = 0; k < 3; ++k)
-#pragma unroll
-                                        for (int j = 0; j < 3; ++j) {
-                                            const R wjk = w[1][j] * w[2][k];
-#pragma unroll
-                                            for (int i = 0; i < 3; ++i)
-                                                sum = fma2(dup2(w[0][i] * wjk), tb[EXT ? pidx(i, j, k) : 0], sum);
-                                        }
-                                    tsum.ts = lo2(sum);
-                                    tsum.ws = hi2(sum);
-                                }
+                        for (int a = 0; a < 3; ++a) {
+                            if (has_lo) {
+                                // (xi, lo) <- xi + (lo + v dt/dx), Knuth's two-sum: exact
+                                const R inc = fma(v[a], dtdx, lo[a]);
+                                const R s = xi[a] + inc;
+                                const R bv = s - xi[a];
+                                lo[a] = (xi[a] - (s - bv)) + (inc - bv);
+                                xi[a] = s;
                             } else {
-                                ++c_esc;
-                                if (EXT && P.heat_on) tsum = gather_T_global<R>(P, gr, g0x, g0y, g0z, xi[0], xi[1], xi[2]);
+                                xi[a] = fma(v[a], dtdx, xi[a]);
                             }
-                            if (EXT && P.heat_on && tsum.ws > R(1e-8)) {
-                                // heat conduction: the temperature gather of mpmG2PKernel
-                                // (src/MPMWorkpieceSolver.cu:282-306), clamped to [Tamb, Tm]
-                                dT = fmin(fmax(tsum.ts / tsum.ws, P.Tamb), P.Tamb + P.dTmax) - P.Tamb;
+                        }
+                        dirtyA = true;
+                        if (st == ST_CHIP) {
+                            edot = R(0);
+                        } else {
+                            // C = factor/dx^2 * B with B = dx (M - d v), then decay (0 in the far zone)
+                            const R cf = far ? R(0) : P.apic * idx_ * P.decay;
+#pragma unroll
+                            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) Cm[a * 3 + c] = cf * (M[a][c] - d[c] * v[a]);
+                            have_C = true;
+                            // F <- (I + L dt) F  as  H <- H + Ldt (I + H)
+                            R Ld[9];
+#pragma unroll
+                            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) Ld[a * 3 + c] = L[a][c] * dtdx;
+                            R Hn[9];
+#pragma unroll
+                            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                                for (int c = 0; c < 3; ++c)
+                                    Hn[a * 3 + c] = H[a * 3 + c] + Ld[a * 3 + c] + Ld[a * 3] * H[c] +
+                                                    Ld[a * 3 + 1] * H[3 + c] + Ld[a * 3 + 2] * H[6 + c];
+#pragma unroll
+                            for (int q = 0; q < 9; ++q) H[q] = Hn[q];
+                            const R l00 = L[0][0] * idx_, l11 = L[1][1] * idx_, l22 = L[2][2] * idx_;
+                            const R s01 = (L[0][1] + L[1][0]) * idx_, s02 = (L[0][2] + L[2][0]) * idx_,
+                                    s12 = (L[1][2] + L[2][1]) * idx_;
+                            edot = sqrt(R(2.0 / 3.0) * (l00 * l00 + l11 * l11 + l22 * l22 + R(0.5) * s01 * s01 +
+                                                          R(0.5) * s02 * s02 + R(0.5) * s12 * s12));
+                        }
+                    }
+                    // adiabatic shear band heating after the move and before chip separation
+                    // (AdiabaticShearModel::update after g2pKernel, src/MPMSolver.cu:1130-1132;
+                    // guards of src/AdiabaticShearModel.cu:114-136); the stress is the one the
+                    // constitutive update of this step stored
+                    if (EXT && P.asb_on) {
+                        if (st == ST_CHIP) {
+                            if (ps.asb[pi] != 0) ps.asb[pi] = 0;   // :114-117
+                        } else if (st == ST_ACTIVE && dT > P.asb_rise) {   // :119-123
+                            if (edot < P.asb_min_rate) {                    // :131-136: decay
+                                const uint8_t c = ps.asb[pi];
+                                if (c != 0) ps.asb[pi] = (uint8_t)(c - 1);
+                            } else {
+                                dT = asb_update<R>(P, ps, pi, edot, dT, ctr);
+                                dirtyA = true;
                             }
+                        }
+                    }
+                    // chip separation and fracture after the move (step counter parity)
+                    if (chip_now) {
+                        if (st == ST_ACTIVE) {
+                            // (the FP64 height only of damaged particles)
+                            if (MPMB_UNLIKELY(Dm > R(1e-6)) &&
+                                P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx <
+                                    ds(da(pose[2], P.tool_tip_dz), dm(P.dx, 1.5))) {
+                                st = ST_CHIP;
+                                const V4<R> s0 = ldcs4(&ps.S[0][pi]);
+                                const R rs = sqrt(s0.x * s0.x + s0.y * s0.y + s0.z * s0.z);
+                                ps.sres[pi] = fmax(ps.sres[pi], rs);
+                                stcs4(&ps.S[0][pi], mk4<R>(0, 0, 0, 0));
+                                stcs4(&ps.S[1][pi], mk4<R>(0, 0, 0, 0));
+                                Dm = fmax(Dm, P.Dth);
+                                dirtyA = true;
+                            }
+                        } else if (MPMB_UNLIKELY(st == ST_CHIP && Dm >= P.Dth * R(1.5))) {
+                            const uint32_t seed = (uint32_t)ps.id[pi] * 2654435761u;
+                            const R rx = (R)((double)((seed >> 16) & 0xFF) / 255.0 - 0.5);
+                            const R ry = (R)((double)((seed >> 8) & 0xFF) / 255.0 - 0.5);
+                            const R rz = (R)((double)(seed & 0xFF) / 255.0 - 0.5);
+                            const R sp = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+                            const R pm = sp * R(0.3) + R(0.5);
+                            v[0] += rx * pm; v[1] += ry * pm; v[2] += rz * pm;
+                            Dm = P.Dth * R(0.5);
+                            dirtyA = true;
+                        }
+                    }
+                    // particle-side tool contact after the move, at the tool pose of the
+                    // step's end (every contact_every-th step)
+                    if (MPMB_UNLIKELY(P.contact_every > 0 && !fixed && ((P.step0 + sa.k + 1) % P.contact_every) == 0)) {
+                        const double te = da(P.t0, dm((double)(sa.k + 1), P.dt));
+                        const double pe0 = da(P.tool_p0[0], dm(P.tool_v[0], ds(te, P.tool_t0)));
+                        const double pe2 = da(P.tool_p0[2], dm(P.tool_v[2], ds(te, P.tool_t0)));
+                        const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx;
+                        const double wz = P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx;
+                        ContactOut co;
+                        if (EXT && P.sdf_on) {
+                            // voxel tool SDF (the extension variant)
+                            const double pe1 = da(P.tool_p0[1], dm(P.tool_v[1], ds(te, P.tool_t0)));
+                            const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx;
+                            co = particle_contact_sdf<R>(P, wx, wy, wz, pe0, pe1, pe2, v[0], v[1], v[2], dT);
+                        } else {
+                            co = particle_contact<R>(P, wx, wz, pe0, pe2, v[0], v[1], v[2], dT);
+                        }
+                        if (co.hit) {
 #pragma unroll
                             for (int a = 0; a < 3; ++a) {
                                 if (has_lo) {
-                                    // (xi, lo) <- xi + (lo + v dt/dx), Knuth's two-sum: exact
-                                    const R inc = fma(v[a], dtdx, lo[a]);
+                                    const R inc = (R)co.dxi[a] + lo[a];
                                     const R s = xi[a] + inc;
                                     const R bv = s - xi[a];
                                     lo[a] = (xi[a] - (s - bv)) + (inc - bv);
                                     xi[a] = s;
                                 } else {
-                                    xi[a] = fma(v[a], dtdx, xi[a]);
+                                    xi[a] = (R)((double)xi[a] + co.dxi[a]);
                                 }
                             }
                             dirtyA = true;
-                            if (st == ST_CHIP) {
-                                edot = R(0);
-                            } else {
-                                // C = factor/dx^2 * B with B = dx (M - d v), then decay (0 in the far zone)
-                                const R cf = far ? R(0) : P.apic * idx_ * P.decay;
-#pragma unroll
-                                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c) Cm[a * 3 + c] = cf * (M[a][c] - d[c] * v[a]);
-                                have_C = true;
-                                // F <- (I + L dt) F  as  H <- H + Ldt (I + H)
-                                R Ld[9];
-#pragma unroll
-                                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c) Ld[a * 3 + c] = L[a][c] * dtdx;
-                                R Hn[9];
-#pragma unroll
-                                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c)
-                                        Hn[a * 3 + c] = H[a * 3 + c] + Ld[a * 3 + c] + Ld[a * 3] * H[c] +
-                                                        Ld[a * 3 + 1] * H[3 + c] + Ld[a * 3 + 2] * H[6 + c];
-#pragma unroll
-                                for (int q = 0; q < 9; ++q) H[q] = Hn[q];
-                                const R l00 = L[0][0] * idx_, l11 = L[1][1] * idx_, l22 = L[2][2] * idx_;
-                                const R s01 = (L[0][1] + L[1][0]) * idx_, s02 = (L[0][2] + L[2][0]) * idx_,
-                                        s12 = (L[1][2] + L[2][1]) * idx_;
-                                edot = sqrt(R(2.0 / 3.0) * (l00 * l00 + l11 * l11 + l22 * l22 + R(0.5) * s01 * s01 +
-                                                              R(0.5) * s02 * s02 + R(0.5) * s12 * s12));
-                            }
+                            ++c_contact;
+                            f_work += co.work;
+                            f_force += co.force;
                         }
-                        // adiabatic shear band heating after the move and before chip separation
-                        // (AdiabaticShearModel::update after g2pKernel, src/MPMSolver.cu:1130-1132;
-                        // guards of src/AdiabaticShearModel.cu:114-136); the stress is the one the
-                        // constitutive update of this step stored
-                        if (EXT && P.asb_on) {
-                            if (st == ST_CHIP) {
-                                if (ps.asb[pi] != 0) ps.asb[pi] = 0;   // :114-117
-                            } else if (st == ST_ACTIVE && dT > P.asb_rise) {   // :119-123
-                                if (edot < P.asb_min_rate) {                    // :131-136: decay
-                                    const uint8_t c = ps.asb[pi];
-                                    if (c != 0) ps.asb[pi] = (uint8_t)(c - 1);
-                                } else {
-                                    dT = asb_update<R>(P, ps, pi, edot, dT, ctr);
-                                    dirtyA = true;
-                                }
-                            }
-                        }
-                        // chip separation and fracture after the move (step counter parity)
-                        if (chip_now) {
-                            if (st == ST_ACTIVE) {
-                                // (the FP64 height only of damaged particles)
-                                if (MPMB_UNLIKELY(Dm > R(1e-6)) &&
-                                    P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx <
-                                        ds(da(pose[2], P.tool_tip_dz), dm(P.dx, 1.5))) {
-                                    st = ST_CHIP;
-                                    const V4<R> s0 = ldcs4(&ps.S[0][pi]);
-                                    const R rs = sqrt(s0.x * s0.x + s0.y * s0.y + s0.z * s0.z);
-                                    ps.sres[pi] = fmax(ps.sres[pi], rs);
-                                    stcs4(&ps.S[0][pi], mk4<R>(0, 0, 0, 0));
-                                    stcs4(&ps.S[1][pi], mk4<R>(0, 0, 0, 0));
-                                    Dm = fmax(Dm, P.Dth);
-                                    dirtyA = true;
-                                }
-                            } else if (MPMB_UNLIKELY(st == ST_CHIP && Dm >= P.Dth * R(1.5))) {
-                                const uint32_t seed = (uint32_t)ps.id[pi] * 2654435761u;
-                                const R rx = (R)((double)((seed >> 16) & 0xFF) / 255.0 - 0.5);
-                                const R ry = (R)((double)((seed >> 8) & 0xFF) / 255.0 - 0.5);
-                                const R rz = (R)((double)(seed & 0xFF) / 255.0 - 0.5);
-                                const R sp = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-                                const R pm = sp * R(0.3) + R(0.5);
-                                v[0] += rx * pm; v[1] += ry * pm; v[2] += rz * pm;
-                                Dm = P.Dth * R(0.5);
-                                dirtyA = true;
-                            }
-                        }
-                        // particle-side tool contact after the move, at the tool pose of the
-                        // step's end (every contact_every-th step)
-                        if (MPMB_UNLIKELY(P.contact_every > 0 && !fixed && ((P.step0 + sa.k + 1) % P.contact_every) == 0)) {
-                            const double te = da(P.t0, dm((double)(sa.k + 1), P.dt));
-                            const double pe0 = da(P.tool_p0[0], dm(P.tool_v[0], ds(te, P.tool_t0)));
-                            const double pe2 = da(P.tool_p0[2], dm(P.tool_v[2], ds(te, P.tool_t0)));
-                            const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx;
-                            const double wz = P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx;
-                            ContactOut co;
-                            if (EXT && P.sdf_on) {
-                                // voxel tool SDF (the extension variant)
-                                const double pe1 = da(P.tool_p0[1], dm(P.tool_v[1], ds(te, P.tool_t0)));
-                                const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx;
-                                co = particle_contact_sdf<R>(P, wx, wy, wz, pe0, pe1, pe2, v[0], v[1], v[2], dT);
-                            } else {
-                                co = particle_contact<R>(P, wx, wz, pe0, pe2, v[0], v[1], v[2], dT);
-                            }
-                            if (co.hit) {
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) {
-                                    if (has_lo) {
-                                        const R inc = (R)co.dxi[a] + lo[a];
-                                        const R s = xi[a] + inc;
-                                        const R bv = s - xi[a];
-                                        lo[a] = (xi[a] - (s - bv)) + (inc - bv);
-                                        xi[a] = s;
-                                    } else {
-                                        xi[a] = (R)((double)xi[a] + co.dxi[a]);
-                                    }
-                                }
-                                dirtyA = true;
-                                ++c_contact;
-                                f_work += co.work;
-                                f_force += co.force;
+                    }
+                } else {
+                    // P2G-only launch: velocity and strain rate come from memory
+                    v[0] = b0_ld.x; v[1] = b0_ld.y; v[2] = b0_ld.z; edot = b0_ld.w;
+                }
+
+                bool yielded = false;
+                // nothing below changes the position's low parts, H0-H7: stored
+                // here, so that they hold no registers through the return
+                if (G2P && dirtyA) {
+                    if (has_lo) stcs4(&ps.X[pi], mk4<R>(lo[0], lo[1], lo[2], R(0)));
+                    stcs4(&ps.A[1][pi], mk4<R>(H[0], H[1], H[2], H[3]));
+                    stcs4(&ps.A[2][pi], mk4<R>(H[4], H[5], H[6], H[7]));
+                }
+                // the head's values are in registers: the next round's may come
+                fetch_head(base + kNT);
+                if (kStage && P2G) async_wait<1>();   // this round's F_p
+                if (P2G) {
+                    // kill zone on the cell index, :130-139.  Written on the floored
+                    // bin-local position so that a NaN position fails every bound and is
+                    // killed, as in the reference, whose integer cell index of a NaN
+                    // position (0 from the GPU's conversion) is below 1; a non-finite
+                    // position also marks the instance's error word (byte 0)
+                    // (the bounds are whole numbers: floor(x) < b exactly when x < b)
+                    const R f0 = xi[0], f1 = xi[1], f2 = xi[2];
+                    const V4<R> bx_ = Sm.kill[0], by_ = Sm.kill[1], bz_ = Sm.kill[2];
+                    if (MPMB_UNLIKELY(!(f0 >= bx_.x && f0 < bx_.y && f1 >= by_.x && f1 < by_.y && f2 >= bz_.x && f2 < bz_.y))) {
+                        if (!isfinite(f0 + f1 + f2)) reinterpret_cast<unsigned char*>(P.ierr)[0] = 1;
+                        st = ST_INACTIVE;
+                        if (G2P) {
+                            // no later G2P writes this particle: store this step's v, strain rate and C
+                            stcs4(&ps.B[0][pi], mk4<R>(v[0], v[1], v[2], edot));
+                            if (have_C) {
+                                stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
+                                stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
+                                stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
                             }
                         }
                     } else {
-                        // P2G-only launch: velocity and strain rate come from memory
-                        v[0] = b0_ld.x; v[1] = b0_ld.y; v[2] = b0_ld.z; edot = b0_ld.w;
-                    }
-
-                    bool yielded = false;
-                    // nothing below changes the position's low parts, H0-H7: stored
-                    // here, so that they hold no registers through the return
-                    if (G2P && dirtyA) {
-                        if (has_lo) stcs4(&ps.X[pi], mk4<R>(lo[0], lo[1], lo[2], R(0)));
-                        stcs4(&ps.A[1][pi], mk4<R>(H[0], H[1], H[2], H[3]));
-                        stcs4(&ps.A[2][pi], mk4<R>(H[4], H[5], H[6], H[7]));
-                    }
-                    // the head's values are in registers: the next round's may come
-                    fetch_head(base + kNT);
-                    if (kStage && P2G) async_wait<1>();   // this round's F_p
-                    if (P2G) {
-                        // kill zone on the cell index, :130-139.  Written on the floored
-                        // bin-local position so that a NaN position fails every bound and is
-                        // killed, as in the reference, whose integer cell index of a NaN
-                        // position (0 from the GPU's conversion) is below 1; a non-finite
-                        // position also marks the instance's error word (byte 0)
-                        // (the bounds are whole numbers: floor(x) < b exactly when x < b)
-                        const R f0 = xi[0], f1 = xi[1], f2 = xi[2];
-                        const V4<R> bx_ = Sm.kill[0], by_ = Sm.kill[1], bz_ = Sm.kill[2];
-                        if (MPMB_UNLIKELY(!(f0 >= bx_.x && f0 < bx_.y && f1 >= by_.x && f1 < by_.y && f2 >= bz_.x && f2 < bz_.y))) {
-                            if (!isfinite(f0 + f1 + f2)) reinterpret_cast<unsigned char*>(P.ierr)[0] = 1;
-                            st = ST_INACTIVE;
-                            if (G2P) {
-                                // no later G2P writes this particle: store this step's v, strain rate and C
-                                stcs4(&ps.B[0][pi], mk4<R>(v[0], v[1], v[2], edot));
-                                if (have_C) {
-                                    stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
-                                    stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
-                                    stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
+                        // within one cell of the kill zone the stress is kept in memory, since a
+                        // kill in the next launch leaves the last computed stress as the state
+                        const bool near_kill = f0 < bx_.z || f0 >= bx_.w || f1 < by_.z || f1 >= by_.w ||
+                                               f2 < bz_.z || f2 >= bz_.w;
+                        bool far = false;
+                        if (MPMB_UNLIKELY(P.lod && st == ST_ACTIVE)) {
+                            const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - pose[3];
+                            const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - pose[4];
+                            const double wz =
+                                P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - (pose[5] + P.tool_tip_dz);
+                            far = sqrt(wx * wx + wy * wy + wz * wz) > P.lod_r2;
+                        }
+                        bool skip = far || fixed || st == ST_CHIP;
+                        R Jv = R(1);
+                        R sig[6] = {0, 0, 0, 0, 0, 0};
+                        R sl[3] = {0, 0, 0};
+                        if (!skip && st == ST_ACTIVE) {
+                            // F_p - I, in the stage since the last round (FP64: loaded
+                            // here), rather than in registers through the gather
+                            const V4<R> a4 = kStage ? Sm.stage[kStage ? 5 : 0][tid] : ldcs4(&ps.A[4][pi]),
+                                        a5 = kStage ? Sm.stage[kStage ? 6 : 0][tid] : ldcs4(&ps.A[5][pi]);
+                            R Hp[9] = {a4.x, a4.y, a4.z, a4.w, a5.x, a5.y, a5.z, a5.w, Hp8};
+                            R bsv[6];
+                            R* bsp = nullptr;
+                            if (MPMB_UNLIKELY(P.Hkin > R(0))) {
+                                const V4<R> k0 = ps.K[0][pi], k1 = ps.K[1][pi];
+                                bsv[0] = k0.x; bsv[1] = k0.y; bsv[2] = k0.z; bsv[3] = k0.w;
+                                bsv[4] = k1.x; bsv[5] = k1.y;
+                                bsp = bsv;
+                            }
+                            JCOut jo = jc_update<R>(P, H, Hp, eps, dT, Dm, edot, sig, sl, Jv, &ps.sres[pi], bsp,
+                                                    errf, wk.inst + 1);
+                            if (MPMB_UNLIKELY(jo.yielded)) {
+                                yielded = true;
+                                dirtyA = true;
+                                Hp8 = Hp[8];
+                                stcs4(&ps.A[4][pi], mk4<R>(Hp[0], Hp[1], Hp[2], Hp[3]));
+                                stcs4(&ps.A[5][pi], mk4<R>(Hp[4], Hp[5], Hp[6], Hp[7]));
+                                if (bsp) {
+                                    ps.K[0][pi] = mk4<R>(bsv[0], bsv[1], bsv[2], bsv[3]);
+                                    ps.K[1][pi] = mk4<R>(bsv[4], bsv[5], R(0), R(0));
                                 }
                             }
-                        } else {
-                            // within one cell of the kill zone the stress is kept in memory, since a
-                            // kill in the next launch leaves the last computed stress as the state
-                            const bool near_kill = f0 < bx_.z || f0 >= bx_.w || f1 < by_.z || f1 >= by_.w ||
-                                                   f2 < bz_.z || f2 >= bz_.w;
-                            bool far = false;
-                            if (MPMB_UNLIKELY(P.lod && st == ST_ACTIVE)) {
-                                const double wx = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - pose[3];
-                                const double wy = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - pose[4];
-                                const double wz =
-                                    P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - (pose[5] + P.tool_tip_dz);
-                                far = sqrt(wx * wx + wy * wy + wz * wz) > P.lod_r2;
+                            if (jo.to_chip) { st = ST_CHIP; skip = true; }
+                            // with the shear model on, the next step's heating reads the stress
+                            // of every particle that passes its temperature guard
+                            if (MPMB_UNLIKELY(sa.sigma_all || Dm > R(1e-6) || P.lod || near_kill ||
+                                              (P.asb_on && dT > P.asb_rise))) {
+                                stcs4(&ps.S[0][pi], mk4<R>(sig[0], sig[1], sig[2], sig[3]));
+                                stcs4(&ps.S[1][pi], mk4<R>(sig[4], sig[5], R(0), R(0)));
                             }
-                            bool skip = far || fixed || st == ST_CHIP;
-                            R Jv = R(1);
-                            R sig[6] = {0, 0, 0, 0, 0, 0};
-                            R sl[3] = {0, 0, 0};
-                            if (!skip && st == ST_ACTIVE) {
-                                // F_p - I, in the stage since the last round (FP64: loaded
-                                // here), rather than in registers through the gather
-                                const V4<R> a4 = kStage ? Sm.stage[kStage ? 5 : 0][tid] : ldcs4(&ps.A[4][pi]),
-                                            a5 = kStage ? Sm.stage[kStage ? 6 : 0][tid] : ldcs4(&ps.A[5][pi]);
-                                R Hp[9] = {a4.x, a4.y, a4.z, a4.w, a5.x, a5.y, a5.z, a5.w, Hp8};
-                                R bsv[6];
-                                R* bsp = nullptr;
-                                if (MPMB_UNLIKELY(P.Hkin > R(0))) {
-                                    const V4<R> k0 = ps.K[0][pi], k1 = ps.K[1][pi];
-                                    bsv[0] = k0.x; bsv[1] = k0.y; bsv[2] = k0.z; bsv[3] = k0.w;
-                                    bsv[4] = k1.x; bsv[5] = k1.y;
-                                    bsp = bsv;
+                        }
+                        // C of the particle: from this launch's gather, or the frozen value of
+                        // a CHIP particle (g2pKernel keeps it)
+                        if (MPMB_UNLIKELY(!have_C && !fixed)) {
+                            const V4<R> c1 = ldcs4(&ps.B[1][pi]), c2 = ldcs4(&ps.B[2][pi]),
+                                        c3 = ldcs4(&ps.B[3][pi]);
+                            Cm[0] = c1.x; Cm[1] = c1.y; Cm[2] = c1.z; Cm[3] = c1.w;
+                            Cm[4] = c2.x; Cm[5] = c2.y; Cm[6] = c2.z; Cm[7] = c2.w; Cm[8] = c3.x;
+                        }
+                        if (MPMB_UNLIKELY(!fixed && have_C && st == ST_CHIP && st_in != ST_CHIP)) {
+                            // turned CHIP this launch: freeze C as the reference does
+                            stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
+                            stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
+                            stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
+                            wrote_C = true;
+                        }
+                        // scatter payload: Q = m (v - dx C d) + f_ext dt, R = m dx C,
+                        // S = -dt V J sigma / dx (sigma with the reference's trial lower triangle)
+                        int bb[3];
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            const R fb = floor(xi[a] - R(0.5));
+                            pay.d[a] = xi[a] - fb;
+                            bb[a] = (int)fb;
+                        }
+                        const R m = P.pmass;
+                        R(&Q)[3] = pay.Q;
+                        R(&Rm)[9] = pay.Rm;
+                        R(&S)[9] = pay.S;
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) Q[q] = R(0);
+#pragma unroll
+                        for (int q = 0; q < 9; ++q) { Rm[q] = R(0); S[q] = R(0); }
+                        R ef[3] = {0, 0, 0};
+                        if (MPMB_UNLIKELY(sa.use_ext && P.pext)) {
+                            // an imported per-particle force (MPMParticle::ext_f) acts on every
+                            // particle the step scatters, FIXED included: p2gKernel adds
+                            // w * ext_f to the node force (src/MPMSolver.cu:410-417)
+                            const V4<R> e = P.pext[P.pbase + ps.orig[pi]];
+                            const R fdt = (R)P.dt;
+                            ef[0] = e.x * fdt; ef[1] = e.y * fdt; ef[2] = e.z * fdt;
+                            if (fixed) { Q[0] = ef[0]; Q[1] = ef[1]; Q[2] = ef[2]; }
+                        }
+                        if (!fixed) {
+                            const R(&d)[3] = pay.d;
+                            const R mdx = m * (R)P.dx;
+                            if (MPMB_UNLIKELY(sa.use_ext && P.ext_r > 0.0 && (st == ST_ACTIVE || st == ST_CHIP))) {
+                                const double ex = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - P.ext_c[0];
+                                const double ey = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - P.ext_c[1];
+                                const double ez = P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - P.ext_c[2];
+                                const double dist = sqrt(ex * ex + ey * ey + ez * ez);
+                                if (dist < P.ext_r) {
+                                    const double fw = (1.0 - dist / P.ext_r) * P.dt;
+                                    ef[0] += (R)(P.ext_f[0] * fw); ef[1] += (R)(P.ext_f[1] * fw);
+                                    ef[2] += (R)(P.ext_f[2] * fw);
                                 }
-                                JCOut jo = jc_update<R>(P, H, Hp, eps, dT, Dm, edot, sig, sl, Jv, &ps.sres[pi], bsp,
-                                                        errf, wk.inst + 1);
-                                if (MPMB_UNLIKELY(jo.yielded)) {
-                                    yielded = true;
-                                    dirtyA = true;
-                                    Hp8 = Hp[8];
-                                    stcs4(&ps.A[4][pi], mk4<R>(Hp[0], Hp[1], Hp[2], Hp[3]));
-                                    stcs4(&ps.A[5][pi], mk4<R>(Hp[4], Hp[5], Hp[6], Hp[7]));
-                                    if (bsp) {
-                                        ps.K[0][pi] = mk4<R>(bsv[0], bsv[1], bsv[2], bsv[3]);
-                                        ps.K[1][pi] = mk4<R>(bsv[4], bsv[5], R(0), R(0));
-                                    }
-                                }
-                                if (jo.to_chip) { st = ST_CHIP; skip = true; }
-                                // with the shear model on, the next step's heating reads the stress
-                                // of every particle that passes its temperature guard
-                                if (MPMB_UNLIKELY(sa.sigma_all || Dm > R(1e-6) || P.lod || near_kill ||
-                                                  (P.asb_on && dT > P.asb_rise))) {
-                                    stcs4(&ps.S[0][pi], mk4<R>(sig[0], sig[1], sig[2], sig[3]));
-                                    stcs4(&ps.S[1][pi], mk4<R>(sig[4], sig[5], R(0), R(0)));
-                                }
                             }
-                            // C of the particle: from this launch's gather, or the frozen value of
-                            // a CHIP particle (g2pKernel keeps it)
-                            if (MPMB_UNLIKELY(!have_C && !fixed)) {
-                                const V4<R> c1 = ldcs4(&ps.B[1][pi]), c2 = ldcs4(&ps.B[2][pi]),
-                                            c3 = ldcs4(&ps.B[3][pi]);
-                                Cm[0] = c1.x; Cm[1] = c1.y; Cm[2] = c1.z; Cm[3] = c1.w;
-                                Cm[4] = c2.x; Cm[5] = c2.y; Cm[6] = c2.z; Cm[7] = c2.w; Cm[8] = c3.x;
-                            }
-                            if (MPMB_UNLIKELY(!fixed && have_C && st == ST_CHIP && st_in != ST_CHIP)) {
-                                // turned CHIP this launch: freeze C as the reference does
-                                stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
-                                stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
-                                stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
-                                wrote_C = true;
-                            }
-                            // scatter payload: Q = m (v - dx C d) + f_ext dt, R = m dx C,
-                            // S = -dt V J sigma / dx (sigma with the reference's trial lower triangle)
-                            int bb[3];
 #pragma unroll
                             for (int a = 0; a < 3; ++a) {
-                                const R fb = floor(xi[a] - R(0.5));
-                                pay.d[a] = xi[a] - fb;
-                                bb[a] = (int)fb;
+                                Q[a] = m * v[a] -
+                                       mdx * (Cm[a * 3] * d[0] + Cm[a * 3 + 1] * d[1] + Cm[a * 3 + 2] * d[2]) + ef[a];
+#pragma unroll
+                                for (int c = 0; c < 3; ++c) Rm[a * 3 + c] = mdx * Cm[a * 3 + c];
                             }
-                            const R m = P.pmass;
-                            R(&Q)[3] = pay.Q;
-                            R(&Rm)[9] = pay.Rm;
-                            R(&S)[9] = pay.S;
-#pragma unroll
-                            for (int q = 0; q < 3; ++q) Q[q] = R(0);
-#pragma unroll
-                            for (int q = 0; q < 9; ++q) { Rm[q] = R(0); S[q] = R(0); }
-                            R ef[3] = {0, 0, 0};
-                            if (MPMB_UNLIKELY(sa.use_ext && P.pext)) {
-                                // an imported per-particle force (MPMParticle::ext_f) acts on every
-                                // particle the step scatters, FIXED included: p2gKernel adds
-                                // w * ext_f to the node force (src/MPMSolver.cu:410-417)
-                                const V4<R> e = P.pext[P.pbase + ps.orig[pi]];
-                                const R fdt = (R)P.dt;
-                                ef[0] = e.x * fdt; ef[1] = e.y * fdt; ef[2] = e.z * fdt;
-                                if (fixed) { Q[0] = ef[0]; Q[1] = ef[1]; Q[2] = ef[2]; }
-                            }
-                            if (!fixed) {
-                                const R(&d)[3] = pay.d;
-                                const R mdx = m * (R)P.dx;
-                                if (MPMB_UNLIKELY(sa.use_ext && P.ext_r > 0.0 && (st == ST_ACTIVE || st == ST_CHIP))) {
-                                    const double ex = P.ox + ((double)g0x + ((double)xi[0] + (double)lo[0])) * P.dx - P.ext_c[0];
-                                    const double ey = P.oy + ((double)g0y + ((double)xi[1] + (double)lo[1])) * P.dx - P.ext_c[1];
-                                    const double ez = P.oz + ((double)g0z + ((double)xi[2] + (double)lo[2])) * P.dx - P.ext_c[2];
-                                    const double dist = sqrt(ex * ex + ey * ey + ez * ez);
-                                    if (dist < P.ext_r) {
-                                        const double fw = (1.0 - dist / P.ext_r) * P.dt;
-                                        ef[0] += (R)(P.ext_f[0] * fw); ef[1] += (R)(P.ext_f[1] * fw);
-                                        ef[2] += (R)(P.ext_f[2] * fw);
-                                    }
-                                }
-#pragma unroll
-                                for (int a = 0; a < 3; ++a) {
-                                    Q[a] = m * v[a] -
-                                           mdx * (Cm[a * 3] * d[0] + Cm[a * 3 + 1] * d[1] + Cm[a * 3 + 2] * d[2]) + ef[a];
-#pragma unroll
-                                    for (int c = 0; c < 3; ++c) Rm[a * 3 + c] = mdx * Cm[a * 3 + c];
-                                }
-                                const R sf = skip ? R(0) : -(R)P.dt * P.pvol * Jv * idx_;
-                                S[0] = sf * sig[0]; S[4] = sf * sig[1]; S[8] = sf * sig[2];
-                                S[1] = sf * sig[3]; S[3] = sf * sl[0];
-                                S[2] = sf * sig[4]; S[6] = sf * sl[1];
-                                S[5] = sf * sig[5]; S[7] = sf * sl[2];
-                            }
-                            if (__builtin_expect(bb[0] >= 0 && bb[0] < kBin && bb[1] >= 0 && bb[1] < kBin && bb[2] >= 0 &&
-                                                     bb[2] < kBin, 1)) {
-                                staged = true;
-                            } else {
-                                off = true;
-                                ++c_esc;
-                            }
-#pragma unroll
-                            for (int a = 0; a < 3; ++a) bc[a] = bb[a];
-                            if (EXT) pay.T = P.Tamb + dT;   // absolute (heat conduction)
+                            const R sf = skip ? R(0) : -(R)P.dt * P.pvol * Jv * idx_;
+                            S[0] = sf * sig[0]; S[4] = sf * sig[1]; S[8] = sf * sig[2];
+                            S[1] = sf * sig[3]; S[3] = sf * sl[0];
+                            S[2] = sf * sig[4]; S[6] = sf * sl[1];
+                            S[5] = sf * sig[5]; S[7] = sf * sl[2];
                         }
-                    }
-
-                    // write back
-                    if (dirtyA) {
-                        stcs4(&ps.A[0][pi], mk4<R>(xi[0], xi[1], xi[2], eps));
-                        stcs4(&ps.A[3][pi], mk4<R>(H[8], Hp8, dT, Dm));
-                    }
-                    if (MPMB_UNLIKELY(st != st_in)) ps.status[pi] = st;
-                    if (G2P && sa.write_out && st != ST_INACTIVE) {
-                        if (fixed) {
-                            const V4<R> b0 = ldcs4(&ps.B[0][pi]);
-                            stcs4(&ps.B[0][pi], mk4<R>(R(0), R(0), R(0), b0.w));
+                        if (__builtin_expect(bb[0] >= 0 && bb[0] < kBin && bb[1] >= 0 && bb[1] < kBin && bb[2] >= 0 &&
+                                                 bb[2] < kBin, 1)) {
+                            staged = true;
                         } else {
-                            stcs4(&ps.B[0][pi], mk4<R>(v[0], v[1], v[2], edot));
-                            if (have_C && !wrote_C && st_in != ST_CHIP) {
-                                stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
-                                stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
-                                stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
-                            }
+                            off = true;
+                            ++c_esc;
+                        }
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) bc[a] = bb[a];
+                        if (EXT) pay.T = P.Tamb + dT;   // absolute (heat conduction)
+                    }
+                }
+
+                // write back
+                if (dirtyA) {
+                    stcs4(&ps.A[0][pi], mk4<R>(xi[0], xi[1], xi[2], eps));
+                    stcs4(&ps.A[3][pi], mk4<R>(H[8], Hp8, dT, Dm));
+                }
+                if (MPMB_UNLIKELY(st != st_in)) ps.status[pi] = st;
+                if (G2P && sa.write_out && st != ST_INACTIVE) {
+                    if (fixed) {
+                        const V4<R> b0 = ldcs4(&ps.B[0][pi]);
+                        stcs4(&ps.B[0][pi], mk4<R>(R(0), R(0), R(0), b0.w));
+                    } else {
+                        stcs4(&ps.B[0][pi], mk4<R>(v[0], v[1], v[2], edot));
+                        if (have_C && !wrote_C && st_in != ST_CHIP) {
+                            stcs4(&ps.B[1][pi], mk4<R>(Cm[0], Cm[1], Cm[2], Cm[3]));
+                            stcs4(&ps.B[2][pi], mk4<R>(Cm[4], Cm[5], Cm[6], Cm[7]));
+                            stcs4(&ps.B[3][pi], mk4<R>(Cm[8], R(0), R(0), R(0)));
                         }
                     }
-                    c_yield += yielded ? 1 : 0;
-                } else {
-                    fetch_head(base + kNT);
-                    if (kStage && P2G) async_wait<1>();
                 }
-                fetch_fp(base + kNT);
-                if (P2G) {
-                    __syncwarp();
-                    for (unsigned far = __ballot_sync(0xffffffffu, off); MPMB_UNLIKELY(far); far &= far - 1u) {
-                        const int e = __ffs((int)far) - 1;
-                        auto from = [&](auto x) { return __shfl_sync(0xffffffffu, x, e); };
-                        Payload<R> p;
+                c_yield += yielded ? 1 : 0;
+            } else {
+                fetch_head(base + kNT);
+                if (kStage && P2G) async_wait<1>();
+            }
+            fetch_fp(base + kNT);
+            if (P2G) {
+                __syncwarp();
+                for (unsigned far = __ballot_sync(0xffffffffu, off); MPMB_UNLIKELY(far); far &= far - 1u) {
+                    const int e = __ffs((int)far) - 1;
+                    auto from = [&](auto x) { return __shfl_sync(0xffffffffu, x, e); };
+                    Payload<R> p;
 #pragma unroll
-                        for (int a = 0; a < 3; ++a) { p.d[a] = from(pay.d[a]); p.Q[a] = from(pay.Q[a]); }
+                    for (int a = 0; a < 3; ++a) { p.d[a] = from(pay.d[a]); p.Q[a] = from(pay.Q[a]); }
 #pragma unroll
-                        for (int q = 0; q < 9; ++q) { p.Rm[q] = from(pay.Rm[q]); p.S[q] = from(pay.S[q]); }
-                        p.T = EXT ? from(pay.T) : R(0);
-                        const int buf = rbuf ^ (G2P ? 1 : 0);
-                        far_scatter<R>(P, gw, EXT && P.heat_on ? P.tm[buf] : nullptr, g0x + from(bc[0]), g0y + from(bc[1]),
-                                       g0z + from(bc[2]), p, P.pmass, lane);
-                    }
-                    __syncwarp();
-                    if (!staged) bc[0] = bc[1] = bc[2] = 0;
-                    warp_scatter<R, EXT>(Sm, wid, lane, staged, bc[0], bc[1], bc[2], pay, P.pmass, P.heat_on != 0);
+                    for (int q = 0; q < 9; ++q) { p.Rm[q] = from(pay.Rm[q]); p.S[q] = from(pay.S[q]); }
+                    p.T = EXT ? from(pay.T) : R(0);
+                    const int buf = rbuf ^ (G2P ? 1 : 0);
+                    far_scatter<R>(P, gw, EXT && P.heat_on ? P.tm[buf] : nullptr, g0x + from(bc[0]), g0y + from(bc[1]),
+                                   g0z + from(bc[2]), p, P.pmass, lane);
                 }
+                __syncwarp();
+                if (!staged) bc[0] = bc[1] = bc[2] = 0;
+                warp_scatter<R, EXT>(Sm, wid, lane, staged, bc[0], bc[1], bc[2], pay, P.pmass, P.heat_on != 0);
+            }
         }
         __syncthreads();   // every warp's adds to its tile
 

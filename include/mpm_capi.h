@@ -508,8 +508,8 @@ typedef struct mpm_launch_config {
      * cover it in a fixed order (no float atomics; one extra launch per step);
      * a particle whose stencil left its bin's tile adds to the grid in 2^-40
      * particle-mass fixed point with integer atomics; and the re-bin's order
-     * within each cell (which it uses in both modes) is the order of the old
-     * slots.  Holds 5 x 216 reals per bin and 5 x 8 bytes per grid node more;
+     * within each cell (which it uses in both modes) is the order of the
+     * upload.  Holds 5 x 216 reals per bin and 5 x 8 bytes per grid node more;
      * every option runs in it (graphs included) except the
      * MPMWorkpieceSolver semantics (MPM_NOT_SUPPORTED at the step). */
     int32_t deterministic;
