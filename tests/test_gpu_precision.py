@@ -13,11 +13,13 @@ particles sit in the damaged corner where the workpiece's free top and end
 faces meet (the impact wave of the tool's first step reflects there), far
 from the tool -- and the chip-fracture decision then adds a velocity kick of
 up to about 1 m/s to one run only.  After such a flip the two runs differ by
-1e-4 to a few 1e-3 in momentum.  On the 64x32x32 case about one seed in three
-flips within 1000 steps; at 128x64x64 every seed tried flips after about 650
-steps.  The tests below pin the target where the decisions agree (the seed of
-the small case; the first 500 steps of the full case) and bound the
-divergence after it.
+1e-4 to a few 1e-3 in momentum.  Which seeds flip depends on the order of the
+FP32 sums, how many do not: on the 64x32x32 case 15 to 18 of 32 runs (16 seeds,
+both returns) end without a flip in four builds with different orders; at
+128x64x64 every seed tried flips after about 650 steps.  So the tests below run
+many seeds, hold every one to the target before the first flips (500 steps),
+compare the size of the rounding errors there, and bound the number of flips
+and what follows them.
 """
 from __future__ import annotations
 
@@ -29,39 +31,61 @@ from mpm_b200 import Solver, capi as A, workpiece as W
 pytestmark = pytest.mark.gpu
 
 
-# placement seed of the small case: FP32 and FP64 take the same decisions through 1000 steps
-SMALL_SEED = 2
+SEEDS = 16
 
 
-def run(case, prec, n):
+def run(case, prec):
+    """Metrics and statuses after 500 and after 1000 steps."""
     b = case["box"]
     s = Solver(W.to_mpm_params(case, precision=prec), int(np.prod(np.subtract(b["c1"], b["c0"]))) * b["ppc"])
     try:
         s.init_box(b["c0"], b["c1"], b["ppc"], b["seed"], 0, b["fixed_layers"], b["T0"], tool=case["tool"])
-        s.step(case["dt"], n)
-        return s.metrics(), s.download(("status",))["status"]
+        out = []
+        for _ in range(2):
+            s.step(case["dt"], 500)
+            out.append((s.metrics(), s.download(("status",))["status"]))
+        return out
     finally:
         s.close()
 
 
+def errors(a, r):
+    """Relative errors of momentum (norm), kinetic + internal energy and peak von Mises stress."""
+    p = np.linalg.norm(np.subtract(a["momentum"], r["momentum"])) / np.linalg.norm(r["momentum"])
+    ea, er = (m["kinetic"] + m["internal_elastic"] for m in (a, r))
+    return np.array([p, abs(ea - er) / er, abs(a["max_von_mises"] - r["max_von_mises"]) / r["max_von_mises"]])
+
+
 @pytest.mark.parametrize("plasticity", [A.PLAST_EXPLICIT, A.PLAST_NEWTON])
-def test_fp32_within_1e4_of_fp64_through_chip_formation(plasticity):
-    case = W.config4(cells=(64, 32, 32))
-    case["box"]["seed"] = SMALL_SEED
-    case["params"]["plasticity"] = plasticity
-    m32, st32 = run(case, A.PREC_F32, 1000)
-    m64, st64 = run(case, A.PREC_F64, 1000)
-    assert m64["n_chip"] > 0   # the run goes through chip separation
-    assert np.array_equal(st32, st64)   # the same threshold decisions
-    p32, p64 = np.array(m32["momentum"]), np.array(m64["momentum"])
-    assert np.linalg.norm(p32 - p64) / np.linalg.norm(p64) <= 1e-4
-    e32 = m32["kinetic"] + m32["internal_elastic"]
-    e64 = m64["kinetic"] + m64["internal_elastic"]
-    assert abs(e32 - e64) / e64 <= 1e-4
-    assert abs(m32["max_von_mises"] - m64["max_von_mises"]) / m64["max_von_mises"] <= 1e-3
-    n = m64["n_active"] + m64["n_chip"] + m64["n_fixed"]
-    assert abs(m32["n_chip"] - m64["n_chip"]) <= max(1, n // 1000)
-    assert abs(m32["mass"] - m64["mass"]) / m64["mass"] <= 1e-6
+def test_fp32_follows_fp64_through_chip_formation(plasticity):
+    early, late, flips = [], [], []
+    for seed in range(SEEDS):
+        case = W.config4(cells=(64, 32, 32))
+        case["box"]["seed"] = seed
+        case["params"]["plasticity"] = plasticity
+        (a, sa), (a2, sa2) = run(case, A.PREC_F32)
+        (r, sr), (r2, sr2) = run(case, A.PREC_F64)
+        assert r2["n_chip"] > 0   # the run goes through chip separation
+        early.append(errors(a, r))
+        late.append(errors(a2, r2))
+        flips.append(int((sa2 != sr2).sum()))
+        # before the first flips: the target, and the same threshold decisions
+        assert np.array_equal(sa, sr), seed
+        assert (early[-1] <= (1e-4, 1e-4, 1e-3)).all(), (seed, early[-1])
+        for x, y in ((a, r), (a2, r2)):
+            assert abs(x["mass"] - y["mass"]) / y["mass"] <= 1e-6
+    early, late, flips = np.array(early), np.array(late), np.array(flips)
+    print(f"\n500 steps: median {np.median(early, 0)}, largest {early.max(0)}; 1000 steps: largest {late.max(0)}, "
+          f"flips {flips.tolist()}")
+    # The size of the rounding errors: the medians over the seeds are 1.7e-7 to 2.1e-7 in every
+    # order of the sums tried, a tenth more or less; a build that lost three bits is above this.
+    assert (np.median(early, 0)[:2] <= 1e-6).all(), early
+    # The flips: 7 to 10 of 16 runs end without one; with a rate of one half, fewer than 3 has a
+    # probability of 2e-3.  At most 23 of 0.51 M particles end with another status, and then the
+    # totals differ by up to 6.7e-3 and 2.5e-3 (bounds: three times what is seen).
+    assert (flips == 0).sum() >= 3, flips
+    assert flips.max() <= 70, flips
+    assert (late.max(0)[:2] <= (2e-2, 7.5e-3)).all(), late
 
 
 def test_config4_full_size_deterministic_fp32():
