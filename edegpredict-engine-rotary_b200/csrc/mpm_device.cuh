@@ -93,7 +93,7 @@ template <typename R> struct alignas(128) Inst {
     R D1, D2, D3, D4c, D5, Dth;
     R Tspan;                       // max(Tm - Tamb, 1)
     R ylo;                         // lower bound of the flow stress of an unheated particle (0: none)
-    R ymin, yslack;                // FlowBound of ylo: ymin (1 - Ts) - yslack, a lower bound at any temperature
+    R ymin;                        // flow_scale of ylo: the lower bound at any temperature is flow_bound(ymin, Ts)
     R dTmax;                       // Tm - Tamb (temperature cap as a rise)
     R heat;                        // beta / max(rho_phys cp, 1e-12)
     R apic;                        // apic_dinv_factor, applied as factor/dx

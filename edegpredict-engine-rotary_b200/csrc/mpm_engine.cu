@@ -742,9 +742,7 @@ class Engine final : public EngineBase {
             d.ylo = (p.jc_A > 0.0 && p.jc_B >= 0.0 && p.jc_C >= 0.0 && rt_lo > 0.0)
                         ? (R)(p.jc_A * rt_lo * (1.0 - 1e-4))
                         : R(0);
-            const FlowBound<R> b = flow_bound<R>(d.ylo, p.jc_m);
-            d.ymin = b.scale;
-            d.yslack = b.slack;
+            d.ymin = flow_scale<R>(d.ylo, p.jc_m);
         }
         d.dTmax = (R)(p.Tm - p.Tamb);
         d.heat = (R)(p.beta / std::max(p.rho_phys * p.cp, 1e-12));

@@ -794,9 +794,9 @@ __device__ __forceinline__ JCOut jc_update(const Inst<R>& P, const R H[9], R Hp[
     // a particle with q below the smallest flow stress the step can have
     // (ylo tt, heated or not: ylo bounds (A + B eps^n)(1 + C ln es) from
     // below, tt = 1 - Ts^m the thermal factor) cannot yield: the flow stress
-    // itself is not needed.  flow_bound_at lies below ylo tt, so most
+    // itself is not needed.  flow_bound lies below ylo tt, so most
     // particles, heated or not, take no power either.
-    if (__builtin_expect(q < flow_bound_at(P.ymin, P.yslack, Ts), 1)) return o;
+    if (__builtin_expect(q < flow_bound(P.ymin, Ts), 1)) return o;
     // (pow(0, y) is +0 for y > 0)
     const R tt = R(1) - ((Ts > R(0) || !(P.m > R(0))) ? pow(Ts, P.m) : R(0));
     if (q < P.ylo * tt) return o;
