@@ -322,6 +322,7 @@ class Engine final : public EngineBase {
         if (p && need <= have) return MPM_OK;
         if (p) cudaFree(p);
         p = nullptr;
+        have = 0;   // (callers that look at the size alone: nothing is there if this fails)
         const int64_t n = headroom ? need + need / 4 : need;
         CK(cudaMalloc(&p, sizeof(T) * n));
         have = n;
@@ -904,7 +905,7 @@ class Engine final : public EngineBase {
             if (s != MPM_OK) return s;
         }
         const size_t need = 4 * (size_t)(2 * ncand + 2 + scan_tmp_size(ncand));
-        if (gen_bytes < need) {
+        if (!d_gen || gen_bytes < need) {
             if (d_gen) cudaFree(d_gen);
             d_gen = nullptr;
             CK(cudaMalloc(&d_gen, need));
@@ -958,7 +959,7 @@ class Engine final : public EngineBase {
         size_t need = 0;
         for (auto& f : fs) need += fbytes(f.src, e, n, (int)f.per);
         need += (h->status ? al256(4 * n) : 0) + (h->id ? al256(4 * n) : 0);
-        if (stage_bytes < need) {
+        if (!d_stage || stage_bytes < need) {
             if (d_stage) cudaFree(d_stage);
             d_stage = nullptr;
             CK(cudaMalloc(&d_stage, need));
@@ -1018,7 +1019,7 @@ class Engine final : public EngineBase {
         size_t need = 0;
         for (auto& f : fs) need += fbytes(f.dst, e, n, (int)f.per);
         need += (h->status ? al256(4 * n) : 0) + (h->id ? al256(4 * n) : 0);
-        if (stage_bytes < need) {
+        if (!d_stage || stage_bytes < need) {
             CK(cudaStreamSynchronize(st));
             if (d_stage) cudaFree(d_stage);
             d_stage = nullptr;
@@ -1058,7 +1059,7 @@ class Engine final : public EngineBase {
         void* out = dst;
         if (!dev) {
             const size_t need = (size_t)504 * std::max<int64_t>(x.np, 1);
-            if (stage_bytes < need) {
+            if (!d_stage || stage_bytes < need) {
                 CK(cudaStreamSynchronize(st));
                 if (d_stage) cudaFree(d_stage);
                 d_stage = nullptr;
@@ -1093,7 +1094,7 @@ class Engine final : public EngineBase {
         const void* in = src;
         if (!dev) {
             const size_t need = (size_t)504 * x.np;
-            if (stage_bytes < need) {
+            if (!d_stage || stage_bytes < need) {
                 CK(cudaStreamSynchronize(st));
                 if (d_stage) cudaFree(d_stage);
                 d_stage = nullptr;
