@@ -80,10 +80,11 @@ __device__ __forceinline__ void async_copy16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// Particle state is read and written once per step: streaming loads and
-// stores (evict-first) keep L1 for the register spills and L2 for the grid
-// tiles and stored node tiles (1.7 % off the fused step on 33.5 M particles,
-// 1.5 % on the 512-workpiece batch).  FP64 keeps plain accesses.
+// Particle state is read and written once per step: FP32 stores, and the loads
+// that do not come through the stage (async_copy16), are streaming ones
+// (evict-first), which keeps L1 for the register spills and L2 for the grid
+// tiles and stored node tiles (1.7 % off the fused step on 33.5 M particles
+// before the stage, when every load was one).  FP64 keeps plain accesses.
 __device__ __forceinline__ float4 ldcs4(const float4* p) { return __ldcs(p); }
 __device__ __forceinline__ D4 ldcs4(const D4* p) { return *p; }
 __device__ __forceinline__ void stcs4(float4* p, const float4 v) { __stcs(p, v); }
@@ -176,8 +177,10 @@ template <> __device__ __forceinline__ void vec_atomic_add<double>(D4* dst, doub
 // Two R values worked on together.  FP32 pairs sit in one 64-bit register and
 // take one instruction (fma.rn.f32x2) for both: the FP32 pipe does no more
 // per cycle than with scalar FMAs (measured 73 against 72 TFLOP/s), but the
-// step kernel is bound by issue slots and their dependency stalls, and a pair
-// takes half of them.  FP64 pairs are two scalar operations.
+// step kernel is bound by the latency of chains of instructions, and a pair
+// halves their number (3.97 -> 3.77 ms on 33.5 M particles, together with the
+// F_p loads and the flow-stress bound of that build).  FP64 pairs are two
+// scalar operations.
 template <typename R> struct alignas(2 * sizeof(R)) P2T { R x, y; };
 template <> struct alignas(8) P2T<float> { unsigned long long v; };
 
@@ -1000,11 +1003,13 @@ __device__ __noinline__ ContactOut particle_contact_sdf(const Inst<R>& P, double
 // ------------------------------------------------------------------ the step kernel
 
 // CTAs per SM the registers are planned for.  The kernel is bound by latency
-// (dependent FMAs, shared-memory round trips, instruction fetches; 44 % of
-// the issue slots used, 17 % of DRAM), so registers trade against warps.
-// FP32: 3 (168 registers a thread): 3.32 ms on 33.5 M particles; 4 (128
-// registers) spills the scatter's coefficients, 4.05 ms.  FP64: 2 (255
-// registers): 277 us on 0.52 M particles where 128 registers took 393 us.
+// (dependent FMAs, shared-memory round trips, instruction fetches; 43 % of
+// the issue slots used, 21 % of DRAM), so registers trade against warps.
+// FP32: 3 (168 registers a thread), 3.32 ms on 33.5 M particles, against 4
+// (128 registers), which spills the scatter's coefficients, 4.05 ms.  FP64: 2
+// (255 registers), 277 us on 0.52 M particles, against 393 us with 128
+// registers.  (Both sides on the builds of that comparison; now 3.35 ms and
+// 207 us.)
 #ifndef MPMB_MIN_CTAS
 #define MPMB_MIN_CTAS 3
 #endif
@@ -1012,9 +1017,9 @@ template <typename R> constexpr int kMinCtas = sizeof(R) == 4 ? MPMB_MIN_CTAS : 
 
 // FP32: each thread's next particle travels to shared memory while it works
 // on the current one (A0-A3, X (P2G-only launches: B0), A4, A5 in the
-// thread's own column of the stage: no barrier, no registers).  With plain
-// loads at the top of the round the kernel waited for DRAM in 1.5 of its 8
-// cycles per issued instruction, with the stage 0.2 of 6.6.
+// thread's own column of the stage: no barrier, no registers).  With loads at
+// the top of the round the kernel waited on L1 and DRAM (long_scoreboard) for
+// 1.76 cycles per issued instruction, with the stage 0.65 of 7.0.
 constexpr int kStageGroups = 7;
 
 // Pairs of a tile's nodes: the 16 lanes of a half warp (x and y 0-3 of one z)
@@ -1089,9 +1094,9 @@ template <typename R> struct PairCoef {
 // (moved since the re-bin, or rows narrower than a warp) wait for a later one,
 // lowest lane first, so the sums have a fixed order.
 // Against the staging of payloads in passes that a thread pair per cell then
-// summed (two CTA barriers a pass, 54 accumulators a thread): 225 M warp
-// instructions instead of 261 M on 4.2 M particles, 3.32 instead of 3.77 ms
-// on 33.5 M (3.97 ms with scalar FMAs).
+// summed (two CTA barriers a pass, 54 accumulators a thread, scalar FMAs): 215 M
+// warp instructions instead of 292 M on 4.2 M particles, 3.35 instead of 3.97
+// ms on 33.5 M.
 template <typename R, bool EXT>
 __device__ __forceinline__ void warp_scatter(StepSmem<R, EXT>& Sm, int wid, int lane, bool staged, int bx, int by,
                                              int bz, const Payload<R>& p, R pm, bool heat) {
@@ -1185,7 +1190,8 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
     // Work items: the first is the CTA's own index, the next ones are drawn from
     // a ticket counter while the current one runs, so that CTAs with light
     // bins (at the workpiece's faces) take more of them: 33.5 M particles 3.28
-    // ms against 3.32 ms in turn, a step of 0.52 M 135 against 140 us.
+    // ms against 3.32 ms with every gridDim-th item, a step of 0.52 M 135
+    // against 140 us.
     for (int wi = blockIdx.x; wi < nw; wi = Sm.next) {
         int drawn = 0;
         if (tid == 0) drawn = (int)gridDim.x + (int)atomicAdd(&ticket[0], 1u);
@@ -1760,7 +1766,9 @@ __global__ void __launch_bounds__(kNT, kMinCtas<R>) k_step(const Inst<R>* __rest
         __syncthreads();   // every warp's adds to its tile
 
         if (P2G) {
-            // end of the bin: its node tile, clearing it for the next bin.
+            // end of the bin: its node tile, clearing it for the next bin.  The
+            // warps' tiles are added in pairs (any fixed order would do: the
+            // results differ in the last bits, their errors do not).
             // Deterministic mode: stored for k_node_sum (every node, zeros
             // included; (m, p) records, then T m); else added to the grid.
             V4<R>* __restrict__ dst = reinterpret_cast<V4<R>*>(static_cast<R*>(sa.part) + (int64_t)wi * kPartReals);
